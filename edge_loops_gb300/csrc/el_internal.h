@@ -77,6 +77,8 @@ el_status launch_thread_mapped(const SpmvCall& c);
 el_status launch_group_mapped(const SpmvCall& c);
 el_status launch_work_oriented(const SpmvCall& c);
 
+// Per B type, defined in spmm_impl.cuh and instantiated in spmm_*.cu.
+template <typename BT> el_status spmm_launch(const SpmmCall& c, int schedule);
 el_status launch_spmm(const SpmmCall& c, int schedule);
 size_t spmm_scratch_bytes(const SpmmCall& c, int schedule);
 long long spmm_slots_needed(const SpmmCall& c, int schedule);

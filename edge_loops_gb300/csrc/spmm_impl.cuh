@@ -1,0 +1,797 @@
+// spmm_impl.cuh -- CSR SpMM C = A B for sm_103a (B, C dense row-major),
+// included once per B type (spmm_f32.cu, spmm_bf16.cu, spmm_f16.cu).
+//
+// One kernel runs the three schedules.  The nonzeros are cut into equal
+// warp ranges along the merge path of row ends and nonzeros, and a warp's
+// range into one PIECE per group of G lanes (G = 4 .. 32, by the width of a
+// B row), so a warp walks 32 / G pieces in step, U nonzeros of each at a
+// time, with the B reads of a step in flight together.  The reads of B are
+// random; what bounds the walk is how many of them the resident warps keep
+// in flight and the instructions between them, so a step waits on nothing
+// else: its columns and values are loaded a step ahead, and the row ends of
+// the range are read once, before the walk, into a bit per nonzero in shared
+// memory.
+//
+//  merge_path: ranges and pieces are cut anywhere; rows that cross pieces
+//    are stitched in shared memory, rows that cross ranges by row-vector
+//    carries that the range where the row ends collects (range ids from an
+//    atomic ticket, bounded spins, fixed order: deterministic).
+//  thread_mapped, group_mapped (ORDERED): cuts are moved to row starts, and
+//    every C element is summed in nonzero order without fused multiply-add,
+//    the reference's order [algorithms/spmm/thread_mapped.cuh:28-53]: equal
+//    bit for bit to the CPU loop.
+// At most 128 columns per pass; wider B is processed in column blocks.
+#pragma once
+
+#include "el_internal.h"
+
+namespace el {
+namespace spmm {
+
+constexpr int kPassCols = 128;  // columns per pass, at most
+constexpr int kWarps = 4;       // per CTA
+constexpr int kTPB = 32 * kWarps;
+constexpr int kBlock = 4096;    // merge items of a range worked on at a time
+constexpr int kMaxNz = 2 * kBlock;  // nonzeros of a block, at most
+// Merge items per row end: a row end costs the walk about two nonzeros (its
+// test, store and new sum).
+constexpr int kRowItems = 2;
+// Resident CTAs per SM: 24 warps of 80 registers (8M nonzeros, n = 32: 187 µs;
+// 20 warps of 96: 205; 32 of 64, which spills in the walk: 230).
+constexpr int kMinCtas = 6;
+
+struct Args {
+  long long rows, cols, nnz;
+  const int* offsets;
+  const int* indices;
+  const unsigned char* values;
+  int value_dtype;
+  const float* row_scale;
+  const unsigned char* B;      // the whole B
+  unsigned long long ldb;      // bytes from one row of B to the next
+  unsigned long long b_first;  // bytes from a row's start to this pass's first column
+  float* C;                    // this pass's first column
+  long long ldc;
+  int n;  // columns in this pass
+  long long range_items;  // merge items per warp
+  int block_items;        // of them worked on at a time, at most kBlock
+  long long num_ranges;
+  WsHeader* hdr;
+  CarrySlot* flags;
+  float* vec;  // num_ranges x kPassCols row-vector carries
+  unsigned long long wait_ns;
+};
+
+// --------------------------------------------------------------- B elements
+template <typename BT>
+__device__ __forceinline__ float bits_to_f32(uint32_t h);
+template <>
+__device__ __forceinline__ float bits_to_f32<float>(uint32_t h) {
+  return __uint_as_float(h);
+}
+template <>
+__device__ __forceinline__ float bits_to_f32<__nv_bfloat16>(uint32_t h) {
+  return __uint_as_float(h << 16);
+}
+template <>
+__device__ __forceinline__ float bits_to_f32<__half>(uint32_t h) {
+  return __half2float(__ushort_as_half((unsigned short)h));
+}
+
+// How a group of G lanes holds a B row: K blocks of V adjacent columns per
+// lane (V elements are one load: rows of B and C start on such boundaries and
+// n is whole vectors; V = 1 takes any alignment and width).
+template <typename BT, int V_, int K_, int G_>
+struct Lay {
+  using T = BT;
+  static constexpr int V = V_, K = K_, G = G_;
+  static constexpr int P = V * K;                           // columns per lane
+  static constexpr int kCols = G * P;                       // columns per group
+  static constexpr int kWords = (V * (int)sizeof(BT) + 3) / 4;  // registers per load
+  static constexpr int U = G < 8 ? G : 8;                   // nonzeros per step
+  static __device__ __forceinline__ int column(int sl, int k) { return V * (sl + G * k); }
+};
+
+// V adjacent elements of a B row, as loaded.
+template <typename L>
+struct BVec {
+  using BT = typename L::T;
+  uint32_t w[L::kWords];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int i = 0; i < L::kWords; ++i) w[i] = 0u;
+  }
+  __device__ __forceinline__ void load(const unsigned char* p) {
+    constexpr int kB = L::V * (int)sizeof(BT);
+    if constexpr (kB == 16) {
+      const uint4 u = __ldg(reinterpret_cast<const uint4*>(p));
+      w[0] = u.x; w[1] = u.y; w[2] = u.z; w[3] = u.w;
+    } else if constexpr (kB == 8) {
+      const uint2 u = __ldg(reinterpret_cast<const uint2*>(p));
+      w[0] = u.x; w[1] = u.y;
+    } else if constexpr (kB == 4) {
+      w[0] = __ldg(reinterpret_cast<const uint32_t*>(p));
+    } else {
+      w[0] = __ldg(reinterpret_cast<const unsigned short*>(p));
+    }
+  }
+  __device__ __forceinline__ float get(int i) const {
+    if (sizeof(BT) == 4) return __uint_as_float(w[i]);
+    return bits_to_f32<BT>((i & 1) ? w[i >> 1] >> 16 : w[i >> 1] & 0xffffu);
+  }
+};
+
+// A nonzero as loaded (nothing waits on the loads before use).
+struct Nz {
+  int c;
+  uint32_t v;  // the value's bits
+  __device__ __forceinline__ void load(const Args& a, bool in, unsigned at) {
+    c = -1;
+    v = 0u;
+    if (in) {
+      c = __ldcs(a.indices + at);
+      if (a.value_dtype == EL_F32)
+        v = __ldcs(reinterpret_cast<const uint32_t*>(a.values) + at);
+      else
+        v = __ldcs(reinterpret_cast<const unsigned short*>(a.values) + at);
+    }
+  }
+  __device__ __forceinline__ float value(const Args& a) const {
+    return a.value_dtype == EL_F32    ? __uint_as_float(v)
+           : a.value_dtype == EL_BF16 ? bits_to_f32<__nv_bfloat16>(v)
+                                      : bits_to_f32<__half>(v);
+  }
+};
+
+template <typename L, bool ORDERED>
+struct Smem {  // per warp
+  static constexpr int NG = 32 / L::G;
+  __align__(16) int idx[2][32];    // a step's columns (-1: none)
+  __align__(16) float val[2][32];  // and values
+  float sc[2][32];                 // scales of the G rows from the step's first on
+  unsigned ends[kMaxNz / 32 + 4];  // bit i: a row ends after the block's nonzero i
+  unsigned rowm[kBlock / 32 + 4];  // bit i: row i of the block ends by such a bit
+  float open[ORDERED ? 1 : NG][ORDERED ? 1 : L::kCols];  // a piece's open row
+  float pend[ORDERED ? 1 : NG][ORDERED ? 1 : L::kCols];  // its part of the row it began inside
+  int first[NG];     // a piece's first row
+  int closed[NG];    // it closed a row
+  int has_pend[NG];  // that first row began before the piece
+};
+
+// bits [at, at + 32) of a bit array
+__device__ __forceinline__ unsigned bits_at(const unsigned* m, int at) {
+  return __funnelshift_r(m[at >> 5], m[(at >> 5) + 1], at & 31);
+}
+
+template <typename L, bool ORDERED>
+struct Walk {
+  using Sm = Smem<L, ORDERED>;
+  static constexpr int G = L::G, U = L::U, NG = 32 / G, P = L::P, V = L::V, K = L::K;
+  const Args& a;
+  Sm& M;
+  const int lane, sl, grp;
+  bool bad_col = false, bad_off = false;
+  const unsigned char* my_B[K];  // the lane's columns of row 0 of B
+
+  __device__ __forceinline__ Walk(const Args& a_, Sm& m_)
+      : a(a_), M(m_), lane(threadIdx.x & 31), sl(lane & (G - 1)), grp(lane / G) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int c = L::column(sl, k);  // past the last column: reads the first again
+      my_B[k] = a.B + a.b_first + (c < a.n ? c : 0) * sizeof(typename L::T);
+    }
+  }
+
+  static __device__ __forceinline__ float mad(float v, float b, float acc) {
+    return ORDERED ? __fadd_rn(acc, __fmul_rn(v, b)) : __fmaf_rn(v, b, acc);
+  }
+  static __device__ __forceinline__ void add(float v, const BVec<L> (&b)[K], float (&acc)[P]) {
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+      for (int i = 0; i < V; ++i) acc[V * k + i] = mad(v, b[k].get(i), acc[V * k + i]);
+  }
+
+  // acc -> the C row whose lane's first column is at dst (streamed: C is not
+  // read again)
+  __device__ __forceinline__ void store(float* dst, const float (&acc)[P], float s) const {
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      if (L::column(sl, k) >= a.n) continue;
+      float* const d = dst + V * G * k;
+      const float* const t = acc + V * k;
+      if constexpr (V == 1)
+        __stcs(d, t[0] * s);
+      else if constexpr (V == 2)
+        __stcs(reinterpret_cast<float2*>(d), make_float2(t[0] * s, t[1] * s));
+      else
+#pragma unroll
+        for (int i = 0; i < V; i += 4)
+          __stcs(reinterpret_cast<float4*>(d + i),
+                 make_float4(t[i] * s, t[i + 1] * s, t[i + 2] * s, t[i + 3] * s));
+    }
+  }
+
+  // The sums of one step: every row end is a store under a predicate.  GAP:
+  // rows skip the empty ones (rw: the rows from the current one on as bits);
+  // SC: rows are scaled.
+  template <bool GAP, bool SC>
+  __device__ __forceinline__ void sums(const BVec<L> (&b)[U][K], const float (&v)[U],
+                                       unsigned ends, unsigned rw, const float* sc,
+                                       float (&acc)[P], float*& crow) const {
+    int moved = 0;
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+      add(v[j], b[j], acc);
+      if ((ends >> j) & 1u) {
+        store(crow, acc, SC ? sc[moved] : 1.f);
+        int gap = 1;
+        if (GAP) {
+          gap = __ffs(rw >> 1);
+          rw >>= gap;
+        }
+        crow += GAP ? gap * a.ldc : a.ldc;
+        if (SC) moved += gap;
+#pragma unroll
+        for (int k = 0; k < P; ++k) acc[k] = 0.f;
+      }
+    }
+  }
+
+  // One block: rows [rs, re) and nonzeros [ns, ne), the rows' ends among
+  // them.  `inside`: row rs began before nonzero ns.  z_out: row rs ends here
+  // without a nonzero.  lone: one row, too long for the bit array, by group 0.
+  // Leaves every piece's open row in M.open, with M.first, closed, has_pend.
+  __device__ __forceinline__ void block(const int rs, const int re, const int ns, const int ne,
+                                        const bool inside, const bool lone, bool& z_out) {
+    const float* const scale = a.row_scale;
+    const int len = ne - ns, nrows = re - rs;
+    // pieces: equal shares of the nonzeros in whole steps (ORDERED: moved to
+    // row starts below)
+    const int per = lone ? len : (len + NG * U - 1) / (NG * U) * U;
+    const long long y0 = ns + (long long)per * grp;
+    int y = y0 < ne ? (int)y0 : ne;
+    int ye = y0 + per < ne ? (int)(y0 + per) : ne;
+    Nz nz;
+    if (!ORDERED || lone) nz.load(a, sl < U && y + sl < ye, y + sl);
+
+    // the row ends as bits; empty rows are written here
+    bool dense = true;
+    z_out = false;
+    if (!lone) {
+      for (int i = lane; i < (len >> 5) + 2; i += 32) M.ends[i] = 0u;
+      for (int i = lane; i < (nrows >> 5) + 2; i += 32) M.rowm[i] = 0u;
+      __syncwarp();
+      for (int i0 = 0; i0 < nrows; i0 += 128) {
+        int s4[4], e4[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = i0 + 32 * u + lane;
+          s4[u] = i < nrows ? __ldg(a.offsets + rs + i) : 0;
+          e4[u] = i < nrows ? __ldg(a.offsets + rs + i + 1) : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (i0 + 32 * u >= nrows) break;
+          const int i = i0 + 32 * u + lane, s = s4[u], e = e4[u];
+          const bool empty = i < nrows && s == e;
+          const bool z = !ORDERED && i == 0 && inside && e == ns;
+          const bool bit = i < nrows && !empty && !z && e > ns && e <= ne;
+          if (bit) {
+            const unsigned m = 1u << ((e - ns - 1) & 31);
+            bad_off |= (atomicOr(&M.ends[(e - ns - 1) >> 5], m) & m) != 0;
+          }
+          bad_off |= i < nrows && !empty && !z && (!bit || e < s || (ORDERED && s < ns));
+          z_out |= __any_sync(kFullMask, z);
+          const unsigned rb = __ballot_sync(kFullMask, bit);
+          if (lane == 0) M.rowm[i >> 5] = rb;
+          dense = dense && rb == __ballot_sync(kFullMask, i < nrows);
+          for (unsigned em = __ballot_sync(kFullMask, empty); em; em &= em - 1) {
+            const long long row = rs + i0 + 32 * u + __ffs(em) - 1;
+            const float zero = scale ? 0.f * __ldg(scale + row) : 0.f;
+            for (int c = lane; c < a.n; c += 32) __stcs(a.C + row * a.ldc + c, zero);
+          }
+        }
+      }
+      __syncwarp();
+    }
+
+    // the row each piece starts in
+    int x = rs;
+    bool began = grp == 0 && inside;
+    if (!lone) {
+      int before = 0;  // the row ends before this group's piece
+#pragma unroll
+      for (int p = 1; p < NG; ++p) {
+        const int q = min(per * p, len);
+        int c = 0;
+        for (int i = lane; i <= q >> 5; i += 32) {
+          unsigned m = M.ends[i];
+          if (i == q >> 5) m &= (1u << (q & 31)) - 1u;
+          c += __popc(m);
+        }
+        c = __reduce_add_sync(kFullMask, c);
+        if (p == grp) before = c;
+      }
+      if (dense) {
+        x = rs + before;
+      } else {
+        // the `before`-th set bit of rowm (re when there is none)
+        int skip = before, at = nrows;
+        for (int i = 0; i <= nrows >> 5; ++i) {
+          const unsigned m = M.rowm[i];
+          const int c = __popc(m);
+          if (skip >= 0 && skip < c) {
+            unsigned t = m;
+            for (int k = 0; k < skip; ++k) t &= t - 1;
+            at = 32 * i + __ffs(t) - 1;
+            skip = -1;
+          } else if (skip >= 0) {
+            skip -= c;
+          }
+        }
+        x = rs + min(at, nrows);
+      }
+      if (ORDERED) {
+        // whole rows: from row x's start to the next piece's row's
+        y = x < re ? min(max(__ldg(a.offsets + x), ns), ne) : ne;
+        ye = __shfl_down_sync(kFullMask, y, G);
+        if (grp == NG - 1) ye = ne;
+        ye = max(y, ye);
+        nz.load(a, sl < U && y + sl < ye, y + sl);
+      } else if (y > ns) {
+        const int q = y - ns - 1;
+        began = !((M.ends[q >> 5] >> (q & 31)) & 1u);
+      } else {
+        began = inside && !z_out;
+      }
+    } else if (grp > 0) {
+      y = ye = ne;
+      x = re;
+    }
+    const int x0 = x;
+    int steps = (ye - y + U - 1) / U;
+#pragma unroll
+    for (int d = G; d < 32; d <<= 1) steps = max(steps, __shfl_xor_sync(kFullMask, steps, d));
+
+    auto step_ends = [&](int at) -> unsigned {  // the piece's row ends in [at, at + U)
+      if (lone || at >= ye) return 0u;
+      const int q = at - ns;
+      if (!ORDERED) {
+        const unsigned b = reinterpret_cast<const unsigned char*>(M.ends)[q >> 3];
+        return U == 8 ? b : (b >> (q & 4)) & 15u;
+      }
+      const int left = ye - at;
+      return bits_at(M.ends, q) & ((1u << (left < U ? left : U)) - 1u);
+    };
+    auto next_row = [&](int r) {  // the next row after r that is not empty
+      int nx = r + 1 - rs;
+      if (!dense) {
+        while (nx < nrows) {
+          const unsigned m = M.rowm[nx >> 5] >> (nx & 31);
+          if (m) {
+            nx += __ffs(m) - 1;
+            break;
+          }
+          nx = (nx & ~31) + 32;
+        }
+        nx = min(nx, nrows);
+      }
+      return rs + nx;
+    };
+    float acc[P];
+#pragma unroll
+    for (int k = 0; k < P; ++k) acc[k] = 0.f;
+    bool has_pend = false;
+    float* crow = a.C + (long long)x * a.ldc + L::column(sl, 0);
+    float scn = scale && !lone ? __ldg(scale + min(x + sl, (int)a.rows - 1)) : 1.f;
+    unsigned ends = step_ends(y);
+#pragma unroll 1
+    for (int i = 0; i < steps; ++i) {
+      const int slot = i & 1;
+      const bool ok = (unsigned)nz.c < (unsigned long long)a.cols;
+      const bool in = y + sl < ye;
+      M.idx[slot][lane] = ok ? nz.c : -1;
+      M.val[slot][lane] = ok ? nz.value(a) : 0.f;
+      if (scale) M.sc[slot][lane] = scn;
+      const bool whole = __all_sync(kFullMask, ok || sl >= U) && a.ldb >> 32 == 0;
+      bad_col |= sl < U && in && !ok;
+      // the next step's loads go first: the B reads of this one are then the
+      // only thing that it waits for
+      nz.load(a, sl < U && y + U + sl < ye, y + U + sl);
+      int xn = x;
+      if (dense)
+        xn += __popc(ends);
+      else if (ends)
+        for (unsigned t = ends; t; t &= t - 1) xn = next_row(xn);
+      if (scale) scn = __ldg(scale + min(xn + sl, (int)a.rows - 1));
+      __syncwarp();
+      BVec<L> b[U][K];
+      if (whole) {
+        int c[U];
+#pragma unroll
+        for (int j = 0; j < U; j += 4) {
+          const int4 t = *reinterpret_cast<const int4*>(&M.idx[slot][grp * G + j]);
+          c[j] = t.x; c[j + 1] = t.y; c[j + 2] = t.z; c[j + 3] = t.w;
+        }
+#pragma unroll
+        for (int j = 0; j < U; ++j)
+#pragma unroll
+          for (int k = 0; k < K; ++k)
+            b[j][k].load(my_B[k] + (unsigned long long)(unsigned)c[j] * (unsigned)a.ldb);
+      } else {
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+          const int c = M.idx[slot][grp * G + j];
+#pragma unroll
+          for (int k = 0; k < K; ++k) {
+            b[j][k].zero();
+            if (c >= 0) b[j][k].load(my_B[k] + (unsigned long long)(unsigned)c * a.ldb);
+          }
+        }
+      }
+      float v[U];
+#pragma unroll
+      for (int j = 0; j < U; j += 4) {
+        const float4 t = *reinterpret_cast<const float4*>(&M.val[slot][grp * G + j]);
+        v[j] = t.x; v[j + 1] = t.y; v[j + 2] = t.z; v[j + 3] = t.w;
+      }
+      const float* const sc = &M.sc[slot][grp * G];
+      if (!__any_sync(kFullMask, ends != 0)) {
+#pragma unroll
+        for (int j = 0; j < U; ++j) add(v[j], b[j], acc);
+      } else {
+        // the first row of a piece may be another's too, and a window of
+        // rows or scales may not reach the last end: those go one by one
+        bool each = ends != 0 && began;
+        unsigned rw = 0u;
+        if (!dense) {
+          rw = bits_at(M.rowm, min(x - rs, nrows));
+          const int ne_ = __popc(ends);
+          each |= ends != 0 && (!(rw & 1u) || __popc(rw) <= ne_ ||
+                                (scale && __popc(rw & (kFullMask >> (32 - G))) < ne_));
+        }
+        if (!__any_sync(kFullMask, each)) {
+          if (dense) {
+            if (scale)
+              sums<false, true>(b, v, ends, 0u, sc, acc, crow);
+            else
+              sums<false, false>(b, v, ends, 0u, sc, acc, crow);
+          } else {
+            if (scale)
+              sums<true, true>(b, v, ends, rw, sc, acc, crow);
+            else
+              sums<true, false>(b, v, ends, rw, sc, acc, crow);
+          }
+        } else {
+          int r = x;
+#pragma unroll 1
+          for (int j = 0; j < U; ++j) {
+            const int c = M.idx[slot][grp * G + j];
+            BVec<L> bj[K];
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+              bj[k].zero();
+              if (c >= 0) bj[k].load(my_B[k] + (unsigned long long)(unsigned)c * a.ldb);
+            }
+            add(M.val[slot][grp * G + j], bj, acc);
+            if ((ends >> j) & 1u) {
+              if (began) {
+                if constexpr (!ORDERED) {
+#pragma unroll
+                  for (int k = 0; k < K; ++k)
+#pragma unroll
+                    for (int t = 0; t < V; ++t)
+                      M.pend[grp][L::column(sl, k) + t] = acc[V * k + t];
+                }
+                has_pend = true;
+                began = false;
+              } else {
+                store(crow, acc, scale ? __ldg(scale + r) : 1.f);
+              }
+#pragma unroll
+              for (int k = 0; k < P; ++k) acc[k] = 0.f;
+              const int nr = next_row(r);
+              crow += (nr - r) * a.ldc;
+              r = nr;
+            }
+          }
+        }
+      }
+      x = xn;
+      y = min(y + U, ye);
+      ends = step_ends(y);
+    }
+    if (lone && grp == 0) store(crow, acc, scale ? __ldg(scale + rs) : 1.f);
+    __syncwarp();
+    if constexpr (!ORDERED) {
+      if (sl == 0) {
+        M.first[grp] = x0;
+        M.closed[grp] = x > x0;
+        M.has_pend[grp] = has_pend;
+      }
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+#pragma unroll
+        for (int t = 0; t < V; ++t) M.open[grp][L::column(sl, k) + t] = acc[V * k + t];
+      __syncwarp();
+    }
+  }
+};
+
+template <typename L, bool ORDERED>
+__global__ void __launch_bounds__(kTPB, kMinCtas) spmm_kernel(const Args a) {
+  using Sm = Smem<L, ORDERED>;
+  constexpr int NG = 32 / L::G;
+  constexpr int Q = (L::kCols + 31) / 32;  // columns per lane when rows are stitched
+  __shared__ Sm smem[kWarps];
+  __shared__ unsigned s_ticket[2];
+  Sm& M = smem[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  long long w = (long long)blockIdx.x * kWarps + (threadIdx.x >> 5);
+  unsigned tag = 0;
+  if (!ORDERED) {
+    // one ticket per CTA: a range only waits on ranges of CTAs that are
+    // running.  The CTA that takes the launch's last ticket hands the
+    // workspace back (every CTA has read the epoch before its ticket).
+    if (threadIdx.x == 0) {
+      const unsigned ep = read_epoch(a.hdr);
+      __threadfence();
+      const unsigned t = atomicAdd(&a.hdr->ticket, 1u);
+      if (t == gridDim.x - 1) {
+        __threadfence();
+        atomicExch(&a.hdr->ticket, 0u);
+        atomicExch(&a.hdr->epoch, ep + 1u);
+      }
+      s_ticket[0] = t;
+      s_ticket[1] = ep;
+    }
+    __syncthreads();
+    w = (long long)s_ticket[0] * kWarps + (threadIdx.x >> 5);
+    tag = epoch_tag(s_ticket[1]);
+  }
+  if (w >= a.num_ranges) return;
+  const long long total = (long long)kRowItems * a.rows + a.nnz;
+  const long long d0 = min(w * a.range_items, total), d1 = min(d0 + a.range_items, total);
+  Walk<L, ORDERED> walk(a, M);
+  float run[Q], pend[Q];  // the open row's partial; row r0's part of this range
+  bool any_closed = false, wait_row = false;  // wait_row: row r0 is ours to finish
+#pragma unroll
+  for (int q = 0; q < Q; ++q) run[q] = pend[q] = 0.f;
+  int r0 = 0, n0 = 0, off_r0 = 0, re = 0, ne = 0, off_re = 0;
+  for (long long d = d0; d < d1; d += a.block_items) {
+    SplitPoint sa, sb;
+    const long long db = min(d + a.block_items, d1);
+    warp_merge_search2_w(a.offsets + 1, a.rows, a.nnz, d, db, kRowItems, sa, sb);
+    auto nz_of = [&](long long dd, const SplitPoint& sp) {  // the nonzero coordinate
+      const long long n = dd - kRowItems * sp.x;
+      return (int)(sp.x < a.rows ? min(n, (long long)sp.end) : n);
+    };
+    int rs = (int)sa.x, ns = nz_of(d, sa);
+    re = (int)sb.x;
+    ne = nz_of(db, sb);
+    off_re = sb.start;
+    bool z = false;
+    if (ORDERED) {  // whole rows
+      const int m = (int)a.nnz;
+      ns = min(max(sa.start, 0), m);
+      ne = min(max(sb.start, ns), m);
+      if (rs < re && ne - ns > kMaxNz) {  // the first of them is longer than a block
+        const int e = min(max(__ldg(a.offsets + rs + 1), ns), ne);
+        walk.block(rs, rs + 1, ns, e, false, true, z);
+        ++rs;
+        ns = e;
+        if (ne - ns > kMaxNz) {  // malformed offsets
+          walk.bad_off = true;
+          ne = ns;
+        }
+      }
+      if (rs < re) walk.block(rs, re, ns, ne, false, false, z);
+    } else {
+      if (d == d0) {
+        r0 = rs;
+        n0 = ns;
+        off_r0 = sa.start;
+      }
+      walk.block(rs, re, ns, ne, ns > sa.start, false, z);
+      // stitch the rows that cross pieces, in piece order
+      const bool need_lb = n0 > off_r0;
+      if (z) {  // row rs ended at the block's first nonzero
+        const float sc = a.row_scale ? __ldg(a.row_scale + rs) : 1.f;
+        const bool lb = need_lb && !any_closed;
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+          const int c = lane + 32 * q;
+          if (lb)
+            pend[q] = run[q];
+          else if (c < a.n)
+            a.C[(long long)rs * a.ldc + c] = run[q] * sc;
+          run[q] = 0.f;
+        }
+        wait_row |= lb;
+        any_closed = true;
+      }
+      for (int s = 0; s < NG; ++s) {
+        const bool hp = M.has_pend[s], cl = M.closed[s], lb = hp && need_lb && !any_closed;
+        const long long row = M.first[s];
+        const float sc = hp && a.row_scale ? __ldg(a.row_scale + row) : 1.f;
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+          const int c = lane + 32 * q;
+          if (c >= a.n) continue;
+          if (hp) {
+            const float t = __fadd_rn(run[q], M.pend[s][c]);
+            if (lb)
+              pend[q] = t;
+            else
+              a.C[row * a.ldc + c] = t * sc;
+          }
+          run[q] = cl ? M.open[s][c] : __fadd_rn(run[q], M.open[s][c]);
+        }
+        wait_row |= lb;
+        any_closed |= cl;
+      }
+      __syncwarp();
+    }
+  }
+  if (walk.bad_off) raise_flag(a.hdr, EL_FLAG_OFFSETS, (unsigned)re);
+  if (walk.bad_col) raise_flag(a.hdr, EL_FLAG_INDEX_RANGE, (unsigned)re);
+  if constexpr (!ORDERED) {
+    // publish the open row's partial vector if this range holds any of it
+    if (re < a.rows && ne > max(off_re, n0)) {
+      float* const dst = a.vec + w * kPassCols;
+#pragma unroll
+      for (int q = 0; q < Q; ++q)
+        if (lane + 32 * q < a.n) __stcg(dst + lane + 32 * q, run[q]);
+      __threadfence();
+      __syncwarp();
+      if (lane == 0) st_release_u32(&a.flags[w].flag, tag);
+    }
+    if (wait_row) {
+      // row r0 began in range `first`: add the partials of ranges [first, w)
+      // in order, 32 flags polled at a time
+      const long long first = max(0LL, ((long long)kRowItems * r0 + off_r0) / a.range_items);
+      float chain[Q];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) chain[q] = 0.f;
+      bool ok = true;
+      for (long long base = first; base < w && ok; base += 32) {
+        if (base + lane < w) {
+          const unsigned* const f = &a.flags[base + lane].flag;
+          if (ld_acquire_u32(f) != tag) {
+            const uint64_t t0 = global_timer_ns();
+            while (ld_acquire_u32(f) != tag) {
+              if (global_timer_ns() - t0 > a.wait_ns) {
+                ok = false;
+                break;
+              }
+              __nanosleep(100);
+            }
+          }
+        }
+        ok = __all_sync(kFullMask, ok);
+        if (!ok) break;
+        const int cnt = (int)(w - base < 32 ? w - base : 32);
+#pragma unroll 8
+        for (int k = 0; k < cnt; ++k) {
+          const float* const src = a.vec + (base + k) * kPassCols;
+#pragma unroll
+          for (int q = 0; q < Q; ++q)
+            if (lane + 32 * q < a.n) chain[q] = __fadd_rn(chain[q], __ldcg(src + lane + 32 * q));
+        }
+        __syncwarp();
+      }
+      if (!ok && lane == 0) raise_flag(a.hdr, EL_FLAG_TIMEOUT, 6);
+      const float sc = a.row_scale ? __ldg(a.row_scale + r0) : 1.f;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int c = lane + 32 * q;
+        if (c < a.n) a.C[(long long)r0 * a.ldc + c] = __fadd_rn(chain[q], pend[q]) * sc;
+      }
+    }
+  }
+}
+
+// ----------------------------------------------------------------- launch
+template <typename L, bool ORDERED>
+el_status launch_kernel(const SpmmCall& c, Args a) {
+  auto kern = spmm_kernel<L, ORDERED>;
+  const int per_sm = resident_ctas_per_sm((const void*)kern, kTPB, 0);
+  long long warps = (long long)(per_sm > 0 ? per_sm : 1) * device_info(c.device).sm_count * kWarps;
+  if (!ORDERED) {
+    const long long most = (long long)(c.scratch_bytes / (kPassCols * sizeof(float)));
+    warps = warps < most ? warps : most;
+    warps = warps < c.ws.nslots ? warps : c.ws.nslots;
+    if (warps < 1) return fail(EL_ERR_INVALID_ARGUMENT, "spmm merge_path: workspace too small");
+  }
+  const long long total = (long long)kRowItems * a.rows + a.nnz;
+  long long ri = (total + warps - 1) / warps;
+  if (ri < 64) ri = 64;
+  a.range_items = ri;
+  const long long blocks = (ri + kBlock - 1) / kBlock;
+  a.block_items = (int)((ri + blocks - 1) / blocks);
+  a.num_ranges = (total + ri - 1) / ri;
+  const long long grid = (a.num_ranges + kWarps - 1) / kWarps;
+  kern<<<(unsigned)grid, kTPB, 0, c.stream>>>(a);
+  return cuda_status(cudaGetLastError(), "spmm launch");
+}
+
+template <typename BT, int V, int K, int G>
+el_status launch_pass(const SpmmCall& c, const Args& a, bool ordered) {
+  using L = Lay<BT, V, K, G>;
+  return ordered ? launch_kernel<L, true>(c, a) : launch_kernel<L, false>(c, a);
+}
+
+template <typename BT>
+el_status launch(const SpmmCall& c, int schedule) {
+  constexpr int kB = (int)sizeof(BT);
+  const bool ordered = schedule != EL_SCHED_MERGE_PATH_FLAT;
+  Args a;
+  a.rows = c.A.rows;
+  a.cols = c.A.cols;
+  a.nnz = c.A.nnz;
+  a.offsets = c.A.offsets;
+  a.indices = c.A.indices;
+  a.values = reinterpret_cast<const unsigned char*>(c.A.values);
+  a.value_dtype = c.A.value_dtype;
+  a.row_scale = c.A.row_scale;
+  a.B = reinterpret_cast<const unsigned char*>(c.B);
+  a.ldb = (unsigned long long)c.ldb * kB;
+  a.ldc = c.ldc;
+  a.hdr = c.ws.hdr;
+  a.flags = c.ws.slots;
+  a.vec = reinterpret_cast<float*>(c.scratch);
+  a.wait_ns = c.wait_ns;
+  // columns per load: the widest vectors on whose boundaries every row of B
+  // and C starts and of which n is a multiple
+  int v = 16 / kB;
+  for (; v > 1; v /= 2) {
+    const int f = v < 4 ? v : 4;  // floats per store
+    if (c.n % v == 0 && c.ldb % v == 0 && (uintptr_t)c.B % (v * kB) == 0 && c.ldc % f == 0 &&
+        (uintptr_t)c.C % (4 * f) == 0)
+      break;
+  }
+  for (long long cb = 0; cb < c.n; cb += kPassCols) {
+    a.n = (int)(c.n - cb < kPassCols ? c.n - cb : kPassCols);
+    a.b_first = (unsigned long long)cb * kB;
+    a.C = c.C + cb;
+    const int n = a.n;
+    el_status s = EL_OK;
+    if (v == 8) {
+      if constexpr (kB == 2)
+        s = n <= 32   ? launch_pass<BT, 8, 1, 4>(c, a, ordered)
+            : n <= 64 ? launch_pass<BT, 8, 1, 8>(c, a, ordered)
+                      : launch_pass<BT, 8, 1, 16>(c, a, ordered);
+    } else if (v == 4) {
+      s = n <= 16   ? launch_pass<BT, 4, 1, 4>(c, a, ordered)
+          : n <= 32 ? launch_pass<BT, 4, 1, 8>(c, a, ordered)
+          : n <= 64 ? launch_pass<BT, 4, 1, 16>(c, a, ordered)
+                    : launch_pass<BT, 4, 1, 32>(c, a, ordered);
+    } else if (v == 2) {
+      s = n <= 16   ? launch_pass<BT, 2, 2, 4>(c, a, ordered)
+          : n <= 32 ? launch_pass<BT, 2, 2, 8>(c, a, ordered)
+          : n <= 64 ? launch_pass<BT, 2, 2, 16>(c, a, ordered)
+                    : launch_pass<BT, 2, 2, 32>(c, a, ordered);
+    } else {
+      s = n <= 8    ? launch_pass<BT, 1, 2, 4>(c, a, ordered)
+          : n <= 16 ? launch_pass<BT, 1, 2, 8>(c, a, ordered)
+          : n <= 32 ? launch_pass<BT, 1, 2, 16>(c, a, ordered)
+          : n <= 64 ? launch_pass<BT, 1, 2, 32>(c, a, ordered)
+          : n <= 96 ? launch_pass<BT, 1, 3, 32>(c, a, ordered)
+                    : launch_pass<BT, 1, 4, 32>(c, a, ordered);
+    }
+    if (s != EL_OK) return s;
+  }
+  return EL_OK;
+}
+
+}  // namespace spmm
+
+template <typename BT>
+el_status spmm_launch(const SpmmCall& c, int schedule) {
+  return spmm::launch<BT>(c, schedule);
+}
+
+#define EL_INSTANTIATE_SPMM(BT) template el_status spmm_launch<BT>(const SpmmCall&, int);
+
+}  // namespace el
