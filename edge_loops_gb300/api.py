@@ -34,9 +34,19 @@ def _ptr(t):
     return None if t is None else C.c_void_p(t.data_ptr())
 
 
+def _raw_stream(stream):
+    """The CUDA stream handle as an int (the current stream for None), read
+    without building a torch.cuda.Stream once CUDA is up: a small call's time
+    is its host time."""
+    if stream is None:
+        if torch.cuda.is_initialized():
+            return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+        stream = torch.cuda.current_stream()
+    return stream.cuda_stream
+
+
 def _stream(stream):
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return C.c_void_p(s.cuda_stream)
+    return C.c_void_p(_raw_stream(stream))
 
 
 def _check_vector(name, t, device, n, dtype=torch.float32):
@@ -50,6 +60,12 @@ def _check_vector(name, t, device, n, dtype=torch.float32):
         raise ValueError(f"{name} must be contiguous")
     if t.numel() < n:
         raise ValueError(f"{name} holds {t.numel()} entries, needs {n}")
+
+
+def _is_vector(t, dev, n):
+    """What _check_vector asks of a float32 vector, on CUDA device `dev`."""
+    return (t.dtype is torch.float32 and t.get_device() == dev and t.is_contiguous()
+            and t.numel() >= n)
 
 
 def _check_on_gpu(A):
@@ -111,14 +127,11 @@ class CSR:
         return self.offsets.device
 
     def el(self):
-        s = L.ElCsr()
-        s.rows, s.cols, s.nnz = self.rows, self.cols, self.nnz
-        s.offsets = self.offsets.data_ptr()
-        s.indices = self.indices.data_ptr() if self.nnz else None
-        s.values = self.values.data_ptr() if self.nnz else None
-        s.value_dtype = _DT[self.values.dtype]
-        s.row_scale = self.row_scale.data_ptr() if self.row_scale is not None else None
-        return s
+        idx, rs = self.indices, self.row_scale
+        nnz = idx.numel()
+        return L.ElCsr(self.rows, self.cols, nnz, self.offsets.data_ptr(),
+                       idx.data_ptr() if nnz else None, self.values.data_ptr() if nnz else None,
+                       _DT[self.values.dtype], 0, rs.data_ptr() if rs is not None else None)
 
     @classmethod
     def from_arrays(cls, offsets, indices, values, cols, device="cuda", rows=None):
@@ -197,8 +210,7 @@ def workspace_errors(ws=None, clear=True, stream=None):
 def make_opts(threads_per_block=0, items_per_thread=0, threads_per_row=0, group_rows=0,
               num_threads=0, compensated=False, max_ctas=0, wait_limit_us=0, variant=0,
               row_weight=0, nz_per_lane=0):
-    o = L.ElSpmvOpts()
-    L.lib().el_spmv_opts_default(C.byref(o))
+    o = L.ElSpmvOpts()  # all zero: el_spmv_opts_default
     o.threads_per_block = threads_per_block
     o.items_per_thread = items_per_thread
     o.threads_per_row = threads_per_row
@@ -216,15 +228,20 @@ def make_opts(threads_per_block=0, items_per_thread=0, threads_per_row=0, group_
 def spmv(A, x, y=None, schedule="merge_path_flat", stream=None, workspace=None, **opts):
     """y = A x (y overwritten), the reference's
     loops::algorithms::spmv::<schedule>(csr, x, y, stream)."""
-    _check_on_gpu(A)
-    _check_vector("x", x, A.device, A.cols)
+    if not A.offsets.is_cuda:
+        _check_on_gpu(A)
+    dev = A.offsets.get_device()
+    if not _is_vector(x, dev, A.cols):
+        _check_vector("x", x, A.device, A.cols)
     if y is None:
         y = torch.empty(A.rows, dtype=torch.float32, device=A.device)
-    _check_vector("y", y, A.device, A.rows)
-    a = A.el()
-    o = make_opts(**opts)
-    L.check(L.lib().el_spmv(_ws(workspace), C.byref(a), _sched(schedule), C.byref(o),
-                            _ptr(x), _ptr(y), _stream(stream)), "el_spmv")
+    elif not _is_vector(y, dev, A.rows):
+        _check_vector("y", y, A.device, A.rows)
+    st = L.lib().el_spmv(_ws(workspace), C.byref(A.el()), _sched(schedule),
+                         C.byref(make_opts(**opts)) if opts else None,
+                         x.data_ptr(), y.data_ptr(), _raw_stream(stream))
+    if st:
+        L.check(st, "el_spmv")
     return y
 
 
@@ -339,11 +356,12 @@ def spmm(A, B, Cm=None, schedule="merge_path_flat", stream=None, workspace=None,
     if Cm.dtype != torch.float32 or Cm.stride(1) != 1 or Cm.shape != (A.rows, n) or \
             Cm.stride(0) < n or Cm.device != A.device:
         raise ValueError("C must be float32 row-major (rows x n) on the matrix's device")
-    a = A.el()
-    o = make_opts(**opts)
-    L.check(L.lib().el_spmm(_ws(workspace), C.byref(a), _sched(schedule), C.byref(o),
-                            _ptr(B), _DT[B.dtype], n, B.stride(0), _ptr(Cm), Cm.stride(0),
-                            _stream(stream)), "el_spmm")
+    st = L.lib().el_spmm(_ws(workspace), C.byref(A.el()), _sched(schedule),
+                         C.byref(make_opts(**opts)) if opts else None,
+                         B.data_ptr(), _DT[B.dtype], n, B.stride(0), Cm.data_ptr(), Cm.stride(0),
+                         _raw_stream(stream))
+    if st:
+        L.check(st, "el_spmm")
     return Cm
 
 
@@ -473,8 +491,9 @@ class BatchPlan:
         return self
 
     def execute(self, stream=None):
-        L.check(L.lib().el_batch_plan_execute(self.handle, _stream(stream)),
-                "el_batch_plan_execute")
+        st = L.lib().el_batch_plan_execute(self.handle, _raw_stream(stream))
+        if st:
+            L.check(st, "el_batch_plan_execute")
 
     def info(self):
         w = C.c_int64()
