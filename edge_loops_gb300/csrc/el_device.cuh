@@ -22,12 +22,12 @@ constexpr unsigned kFullMask = 0xffffffffu;
 // mistaken for fresh ones.  The last CTA (or warp) of a launch resets the
 // ticket and done counters and advances the epoch, all on the device, so a
 // launch can be replayed from a CUDA graph without host-side bookkeeping.
-struct WsHeader {
+struct __align__(16) WsHeader {
   unsigned int ticket;    // next range/tile id handed out
-  unsigned int done;      // CTAs finished (the last one resets both)
+  unsigned int epoch;     // launches completed on this workspace
   unsigned int errors;    // EL_FLAG_* bits, sticky until cleared
   unsigned int err_info;  // first offending index (diagnostics)
-  unsigned int epoch;     // launches completed on this workspace
+  unsigned int done;      // CTAs finished (the last one resets ticket and done)
   unsigned int pad[11];
 };
 static_assert(sizeof(WsHeader) == 64, "header is one 64-byte line");
@@ -55,6 +55,18 @@ __device__ __forceinline__ void finish_launch(WsHeader* h, unsigned epoch) {
   atomicExch(&h->done, 0u);
   atomicExch(&h->epoch, epoch + 1u);
   __threadfence();
+}
+
+// Takes a ticket and reads the epoch in one atomic (they share an aligned
+// 8-byte word).  The launch's last ticket (of `total`) hands the workspace
+// back for the next launch at once: ticket 0, epoch + 1.
+__device__ __forceinline__ void take_ticket(WsHeader* h, unsigned total, unsigned* ticket,
+                                            unsigned* epoch) {
+  unsigned long long* const word = reinterpret_cast<unsigned long long*>(&h->ticket);
+  const unsigned long long v = atomicAdd(word, 1ull);
+  *ticket = (unsigned)v;
+  *epoch = (unsigned)(v >> 32);
+  if (*ticket == total - 1) atomicAdd(word, (1ull << 32) - total);
 }
 
 struct WsView {
@@ -319,10 +331,11 @@ struct SplitPoint {
   int start;    // offsets[x]
   int end;      // offsets[x + 1] (nnz for x == rows)
 };
-__device__ __forceinline__ void warp_merge_search2_w(const int* __restrict__ row_end,
-                                                     long long rows, long long nnz,
-                                                     long long da, long long db, long long w,
-                                                     SplitPoint& A, SplitPoint& B) {
+// `row_end(k)` reads offsets[k + 1], k >= -1.
+template <typename RowEnd>
+__device__ __forceinline__ void warp_merge_search2_w(const RowEnd& row_end, long long rows,
+                                                     long long nnz, long long da, long long db,
+                                                     long long w, SplitPoint& A, SplitPoint& B) {
   const int lane = threadIdx.x & 31;
   long long lo[2], hi[2];
   const long long d[2] = {da, db};
@@ -339,7 +352,7 @@ __device__ __forceinline__ void warp_merge_search2_w(const int* __restrict__ row
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
       p[k] = lo[k] + ((long long)(lane + 1) * (hi[k] - lo[k])) / 33;
-      v[k] = hi[k] - lo[k] > 32 ? __ldg(row_end + p[k]) : 0;  // both loads before either use
+      v[k] = hi[k] - lo[k] > 32 ? row_end(p[k]) : 0;  // both loads before either use
     }
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
@@ -357,7 +370,7 @@ __device__ __forceinline__ void warp_merge_search2_w(const int* __restrict__ row
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
     p[k] = lo[k] + lane;
-    v[k] = p[k] < hi[k] ? __ldg(row_end + p[k]) : 0;
+    v[k] = p[k] < hi[k] ? row_end(p[k]) : 0;
   }
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
@@ -369,8 +382,8 @@ __device__ __forceinline__ void warp_merge_search2_w(const int* __restrict__ row
     // = row_end[x - 1] by lane c - 1 (if c > 0)
     const int ve = __shfl_sync(kFullMask, v[k], c < 32 ? c : 31);
     const int vs = __shfl_sync(kFullMask, v[k], c > 0 ? c - 1 : 0);
-    S.end = (S.x < hi[k] && c < 32) ? ve : S.x < rows ? __ldg(row_end + S.x) : (int)nnz;
-    S.start = c > 0 ? vs : S.x > 0 ? __ldg(row_end + S.x - 1) : __ldg(row_end - 1);
+    S.end = (S.x < hi[k] && c < 32) ? ve : S.x < rows ? row_end(S.x) : (int)nnz;
+    S.start = c > 0 ? vs : S.x > 0 ? row_end(S.x - 1) : row_end(-1);
   }
 }
 

@@ -532,20 +532,8 @@ __global__ void __launch_bounds__(kTPB, kMinCtas) spmm_kernel(const Args a) {
   unsigned tag = 0;
   if (!ORDERED) {
     // one ticket per CTA: a range only waits on ranges of CTAs that are
-    // running.  The CTA that takes the launch's last ticket hands the
-    // workspace back (every CTA has read the epoch before its ticket).
-    if (threadIdx.x == 0) {
-      const unsigned ep = read_epoch(a.hdr);
-      __threadfence();
-      const unsigned t = atomicAdd(&a.hdr->ticket, 1u);
-      if (t == gridDim.x - 1) {
-        __threadfence();
-        atomicExch(&a.hdr->ticket, 0u);
-        atomicExch(&a.hdr->epoch, ep + 1u);
-      }
-      s_ticket[0] = t;
-      s_ticket[1] = ep;
-    }
+    // running
+    if (threadIdx.x == 0) take_ticket(a.hdr, gridDim.x, &s_ticket[0], &s_ticket[1]);
     __syncthreads();
     w = (long long)s_ticket[0] * kWarps + (threadIdx.x >> 5);
     tag = epoch_tag(s_ticket[1]);
@@ -562,7 +550,8 @@ __global__ void __launch_bounds__(kTPB, kMinCtas) spmm_kernel(const Args a) {
   for (long long d = d0; d < d1; d += a.block_items) {
     SplitPoint sa, sb;
     const long long db = min(d + a.block_items, d1);
-    warp_merge_search2_w(a.offsets + 1, a.rows, a.nnz, d, db, kRowItems, sa, sb);
+    warp_merge_search2_w([&](long long k) { return __ldg(a.offsets + 1 + k); }, a.rows, a.nnz, d,
+                         db, kRowItems, sa, sb);
     auto nz_of = [&](long long dd, const SplitPoint& sp) {  // the nonzero coordinate
       const long long n = dd - kRowItems * sp.x;
       return (int)(sp.x < a.rows ? min(n, (long long)sp.end) : n);

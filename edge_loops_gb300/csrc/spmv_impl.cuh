@@ -5,6 +5,7 @@
 
 #include "spmv_merge_path.cuh"
 #include "spmv_merge_path_nz.cuh"
+#include "spmv_merge_path_small.cuh"
 #include "spmv_merge_path_warp.cuh"
 #include "spmv_schedules.cuh"
 

@@ -505,6 +505,47 @@ struct NzWalkK {
 };
 using NzWalk = NzWalkK<kPer>;
 
+// The sum of the partials that ranges [gfirst, g) published of the row they
+// leave open, in a fixed order (a warp's work; bounded waits: ok = false when
+// one ran out).
+template <bool COMP>
+__device__ __forceinline__ Acc<COMP> look_back(const Args& a, long long gfirst, long long g,
+                                               unsigned tag, bool& ok) {
+  const int lane = threadIdx.x & 31;
+  Acc<COMP> acc;
+  ok = true;
+  if (gfirst < 0) gfirst = 0;  // malformed offsets
+  for (long long kk = gfirst + lane; kk < g && kk < a.ws.nslots; kk += 32) {
+    CarrySlot* sl = a.ws.slots + kk;
+    if (ld_acquire_u32(&sl->flag) != tag) {
+      const uint64_t t0 = global_timer_ns();
+      while (ld_acquire_u32(&sl->flag) != tag) {
+        if (global_timer_ns() - t0 > a.wait_ns) {
+          ok = false;
+          break;
+        }
+        __nanosleep(100);
+      }
+    }
+    if (!ok) break;
+    Acc<COMP> pv;
+    pv.set(__ldcg(&sl->sum), __ldcg(&sl->comp));
+    acc.add(pv);
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) {
+    Acc<COMP> ov = shfl_xor_acc(acc, d);
+    if ((lane & d) == 0) {
+      acc.add(ov);
+    } else {
+      ov.add(acc);
+      acc = ov;
+    }
+  }
+  ok = __all_sync(kFullMask, ok);
+  return acc;
+}
+
 // One warp's merge range, shared by the merge-path kernels: takes a range
 // id from the ticket, finds its split points, walks it with `Walk`
 // (rows ending inside are written), publishes the partial of the row left
@@ -519,23 +560,9 @@ __device__ __forceinline__ void run_range(const Args& a, SmemT& S, const int war
 
   // one ticket per CTA (its warps take ranges ticket * warps_per_cta + w):
   // a range only waits on ranges of CTAs that took their ticket earlier and
-  // are therefore running.  Every CTA reads the epoch before its ticket, so
-  // the CTA that takes the launch's last ticket knows that all of them hold
-  // theirs and hands the workspace back for the next launch right away
-  // (ticket to 0, epoch + 1) instead of a completion count at the end.
+  // are therefore running
   __shared__ unsigned s_ticket[2];
-  if (threadIdx.x == 0) {
-    const unsigned ep = read_epoch(hdr);
-    __threadfence();
-    const unsigned t = atomicAdd(&hdr->ticket, 1u);
-    if (t == gridDim.x - 1) {
-      __threadfence();
-      atomicExch(&hdr->ticket, 0u);
-      atomicExch(&hdr->epoch, ep + 1u);
-    }
-    s_ticket[0] = t;
-    s_ticket[1] = ep;
-  }
+  if (threadIdx.x == 0) take_ticket(hdr, gridDim.x, &s_ticket[0], &s_ticket[1]);
   __syncthreads();
   const long long g = (long long)s_ticket[0] * warps_per_cta + (threadIdx.x >> 5);
   const unsigned epoch = s_ticket[1];
@@ -550,7 +577,8 @@ __device__ __forceinline__ void run_range(const Args& a, SmemT& S, const int war
     const long long d0 = dd0 < total ? dd0 : total;
     const long long d1 = dd0 + a.range_items < total ? dd0 + a.range_items : total;
     SplitPoint sa, sb;
-    warp_merge_search2_w(a.offsets + 1, a.rows, a.nnz, d0, d1, w, sa, sb);
+    warp_merge_search2_w([&](long long k) { return __ldg(a.offsets + 1 + k); }, a.rows, a.nnz, d0,
+                         d1, w, sa, sb);
     auto nz_of = [&](long long d, const SplitPoint& sp) {  // the nonzero coordinate
       const long long n = d - w * sp.x;
       return (int)(sp.x < a.rows ? min(n, (long long)sp.end) : n);
@@ -600,39 +628,9 @@ __device__ __forceinline__ void run_range(const Args& a, SmemT& S, const int war
     }
     __syncwarp();
     if (need_lb && S.pend) {
-      // row rs began in range gfirst: sum the partials of ranges [gfirst, g)
-      // in a fixed order
-      const long long gfirst = (w * rs + off_rs) / a.range_items;
-      Acc<COMP> acc;
-      bool ok = true;
-      for (long long kk = gfirst + lane; kk < g && kk < a.ws.nslots; kk += 32) {
-        CarrySlot* sl = a.ws.slots + kk;
-        if (ld_acquire_u32(&sl->flag) != tag) {
-          const uint64_t t0 = global_timer_ns();
-          while (ld_acquire_u32(&sl->flag) != tag) {
-            if (global_timer_ns() - t0 > a.wait_ns) {
-              ok = false;
-              break;
-            }
-            __nanosleep(100);
-          }
-        }
-        if (!ok) break;
-        Acc<COMP> pv;
-        pv.set(__ldcg(&sl->sum), __ldcg(&sl->comp));
-        acc.add(pv);
-      }
-#pragma unroll
-      for (int d = 16; d > 0; d >>= 1) {
-        Acc<COMP> ov = shfl_xor_acc(acc, d);
-        if ((lane & d) == 0) {
-          acc.add(ov);
-        } else {
-          ov.add(acc);
-          acc = ov;
-        }
-      }
-      ok = __all_sync(kFullMask, ok);
+      // row rs began in an earlier range
+      bool ok;
+      Acc<COMP> acc = look_back<COMP>(a, (w * rs + off_rs) / a.range_items, g, tag, ok);
       if (lane == 0) {
         if (!ok) raise_flag(hdr, EL_FLAG_TIMEOUT, 4);
         Acc<COMP> pend;
@@ -690,8 +688,14 @@ inline int nz_per_lane(const SpmvCall& c, int vbytes) {
 template <typename VT, bool COMP, int KP>
 el_status launch_kp(const SpmvCall& c);
 
+template <typename VT>
+bool small_fits(const SpmvCall& c);
+template <typename VT>
+el_status launch_small(const SpmvCall& c);
+
 template <typename VT, bool COMP>
 el_status launch(const SpmvCall& c) {
+  if (!COMP && small_fits<VT>(c)) return launch_small<VT>(c);
   if (c.o.nz_per_lane != 0 && c.o.nz_per_lane != 8 && c.o.nz_per_lane != 16)
     return fail(EL_ERR_INVALID_ARGUMENT, "nz_per_lane must be 0, 8 or 16");
   return nz_per_lane(c, (int)sizeof(VT)) == 16 ? launch_kp<VT, COMP, 16>(c)

@@ -102,9 +102,11 @@ extern "C" el_status el_spmv_static_scratch(const el_csr* A, const float* x, flo
   el_status s = static_scratch(&scratch);
   if (s != EL_OK) return s;
   cudaStream_t st = (cudaStream_t)stream;
-  // ticket, finished counter, error flags and their info start at zero each
-  // call (the epoch is kept: carries of earlier calls never match it)
-  e = cudaMemsetAsync(scratch, 0, 4 * sizeof(unsigned), st);
+  // error flags and their info start at zero each call (the ticket is back at
+  // zero after every launch; the epoch is kept: carries of earlier calls
+  // never match it)
+  e = cudaMemsetAsync(static_cast<char*>(scratch) + offsetof(WsHeader, errors), 0,
+                      2 * sizeof(unsigned), st);
   if (e != cudaSuccess) return cuda_status(e, "clearing the static scratch header");
   switch (A->value_dtype) {
     case EL_F32: s = launch_static<float>(*A, x, y, num_ranges, scratch, device, st); break;
