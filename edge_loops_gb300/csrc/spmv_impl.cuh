@@ -3,6 +3,7 @@
 // the heavy template instantiations compile in parallel.
 #pragma once
 
+#include "spmv_group_mapped.cuh"
 #include "spmv_merge_path.cuh"
 #include "spmv_merge_path_nz.cuh"
 #include "spmv_merge_path_small.cuh"
@@ -122,24 +123,12 @@ struct SpmvImpl {
     return c.o.compensated ? tm_tpr<true>(c) : tm_tpr<false>(c);
   }
 
-  template <int GT, int TPB, bool COMP>
-  static el_status gm(const SpmvCall& c) {
-    constexpr int NG = TPB / GT;
-    const long long groups = (c.A.rows + GT - 1) / GT;
-    long long grid = (groups + NG - 1) / NG;
-    const long long cap = (long long)device_info(c.device).sm_count * 32;
-    if (grid > cap) grid = cap;
-    if (grid < 1) grid = 1;
-    group_mapped_spmv_kernel<VT, GT, TPB, COMP><<<(unsigned)grid, TPB, 0, c.stream>>>(basic(c));
-    return cuda_status(cudaGetLastError(), "group_mapped launch");
-  }
   template <bool COMP>
   static el_status gm_cfg(const SpmvCall& c) {
     const int tpb = c.o.threads_per_block > 0 ? c.o.threads_per_block : 128;
     const int rows = c.o.group_rows > 0 ? c.o.group_rows : tpb;
-    if (rows == 32) return gm<32, 256, COMP>(c);
-    if (rows == 128 && tpb == 128) return gm<128, 128, COMP>(c);
-    if (rows == 256 && tpb == 256) return gm<256, 256, COMP>(c);
+    if (rows == 32 || (rows == 128 && tpb == 128) || (rows == 256 && tpb == 256))
+      return mpn::launch_group_mapped_rows<VT, COMP>(c, rows);
     return fail(EL_ERR_INVALID_ARGUMENT,
                 "group_mapped: group_rows 32 (warp groups) or == threads_per_block "
                 "in {128, 256}");
@@ -148,55 +137,29 @@ struct SpmvImpl {
     return c.o.compensated ? gm_cfg<true>(c) : gm_cfg<false>(c);
   }
 
+  // work_oriented: the reference's even share ceil((rows + nnz) /
+  // num_threads) of the merge path per thread [include/loops/schedule/
+  // work_oriented.hxx:141-195], a warp's 32 shares walked together by the
+  // merge-path walk (row ends and nonzeros count one item each).  By default
+  // one share of 32 threads per resident warp.
   static constexpr int kWoTpb = 128;
-  static constexpr long long kWoShare = 256;    // merge items per thread aimed at
-  static constexpr long long kWoMinShare = 32;  // merge items per thread, at least
-  static constexpr int kWoBlocksPerSm = 16;     // at most this many blocks per SM
-  static long long wo_num_threads(const SpmvCall& c) {
-    if (c.o.num_threads > 0) return c.o.num_threads;
-    // The reference launches 2 x SM count blocks of 128, so each thread walks
-    // thousands of items one latency chain at a time.  Here: every resident
-    // block, and more (one thread per kWoShare items, up to kWoBlocksPerSm
-    // blocks per SM) on large merges -- blocks take their ids from a ticket,
-    // so a look-back only waits on blocks already running -- but no thread
-    // with fewer than kWoMinShare items, since each share pays two global
-    // merge-path searches.
-    const long long blk_items = kWoShare * kWoTpb, min_items = kWoMinShare * kWoTpb;
-    const long long total = c.A.rows + c.A.nnz;
-    const long long sms = device_info(c.device).sm_count;
-    const void* k = c.o.compensated ? (const void*)work_oriented_spmv_kernel<VT, kWoTpb, true>
-                                    : (const void*)work_oriented_spmv_kernel<VT, kWoTpb, false>;
-    const int per_sm = resident_ctas_per_sm(k, kWoTpb, 0);
-    long long nb = (long long)(per_sm > 2 ? per_sm : 2) * sms;
-    const long long share = (total + blk_items - 1) / blk_items;
-    if (share > nb) nb = share;
-    if (nb > kWoBlocksPerSm * sms) nb = kWoBlocksPerSm * sms;
-    const long long most = (total + min_items - 1) / min_items;
-    if (nb > most) nb = most;
-    if (nb < 1) nb = 1;
-    return nb * kWoTpb;
-  }
   static long long work_oriented_slots(const SpmvCall& c) {
-    return (wo_num_threads(c) + kWoTpb - 1) / kWoTpb;
+    const long long m = c.o.compensated ? mpn::slots_needed<VT, true>(c)
+                                        : mpn::slots_needed<VT, false>(c);
+    const long long n = (c.o.num_threads + 31) / 32;
+    return n > m ? n : m;
   }
   template <bool COMP>
   static el_status wo(const SpmvCall& c) {
-    const long long nt = wo_num_threads(c);
-    if (nt % kWoTpb != 0)
+    if (c.o.num_threads > 0 && c.o.num_threads % kWoTpb != 0)
       return fail(EL_ERR_INVALID_ARGUMENT, "work_oriented: num_threads must be a multiple of %d",
                   kWoTpb);
-    WoArgs w;
-    w.b = basic(c);
-    const long long total = c.A.rows + c.A.nnz;
-    w.wpt = (total + nt - 1) / nt;
-    if (w.wpt < 1) w.wpt = 1;
-    w.num_blocks = (int)(nt / kWoTpb);
-    w.wait_ns = c.wait_ns;
-    w.ws = c.ws;
-    if (w.num_blocks > c.ws.nslots)
-      return fail(EL_ERR_INVALID_ARGUMENT, "work_oriented: workspace too small");
-    work_oriented_spmv_kernel<VT, kWoTpb, COMP><<<w.num_blocks, kWoTpb, 0, c.stream>>>(w);
-    return cuda_status(cudaGetLastError(), "work_oriented launch");
+    SpmvCall e = c;
+    e.o.row_weight = 1;
+    e.o.max_ctas = e.o.nz_per_lane = 0;
+    e.trace = nullptr;
+    if (c.o.num_threads > 0) return mpn::launch_shares<VT, COMP>(e, c.o.num_threads);
+    return mpn::launch<VT, COMP>(e);
   }
   static el_status work_oriented(const SpmvCall& c) {
     return c.o.compensated ? wo<true>(c) : wo<false>(c);

@@ -702,17 +702,11 @@ el_status launch(const SpmvCall& c) {
                                                : launch_kp<VT, COMP, 8>(c);
 }
 
+// Launches the walk over ranges of range_items merge items, a row end
+// counted as rw of them.
 template <typename VT, bool COMP, int KP>
-el_status launch_kp(const SpmvCall& c) {
-  const int rw = row_weight(c);
+el_status launch_ranges(const SpmvCall& c, int rw, long long range_items) {
   const long long total = (long long)rw * c.A.rows + c.A.nnz;
-  // ranges of whole 256-item units, one per resident warp
-  const long long units = (total + kTileNz - 1) / kTileNz;
-  long long W = resident_warps<VT, COMP, KP>(c.device);
-  if (c.o.max_ctas > 0 && (long long)c.o.max_ctas * kWarps < W) W = (long long)c.o.max_ctas * kWarps;
-  if (W > units) W = units;
-  if (W < 1) W = 1;
-  const long long upr = (units + W - 1) / W;
   Args a;
   a.rows = c.A.rows;
   a.cols = c.A.cols;
@@ -723,8 +717,8 @@ el_status launch_kp(const SpmvCall& c) {
   a.row_scale = c.A.row_scale;
   a.x = c.x;
   a.y = c.y;
-  a.range_items = upr * kTileNz;
-  a.num_ranges = (units + upr - 1) / upr;
+  a.range_items = range_items;
+  a.num_ranges = (total + range_items - 1) / range_items;
   tile_phase(c.A.indices, c.A.values, (int)sizeof(VT), &a.vec_ok, &a.ph, Geom<KP>::tile);
   a.rw = rw;
   a.test_hooks = c.o.test_hooks;
@@ -737,6 +731,26 @@ el_status launch_kp(const SpmvCall& c) {
   const long long grid = (a.num_ranges + kWarps - 1) / kWarps;
   merge_path_nz_kernel<VT, COMP, KP><<<(unsigned)grid, kTPB, 0, c.stream>>>(a);
   return cuda_status(cudaGetLastError(), "merge_path launch");
+}
+
+template <typename VT, bool COMP, int KP>
+el_status launch_kp(const SpmvCall& c) {
+  const int rw = row_weight(c);
+  const long long total = (long long)rw * c.A.rows + c.A.nnz;
+  // ranges of whole 256-item units, one per resident warp
+  const long long units = (total + kTileNz - 1) / kTileNz;
+  long long W = resident_warps<VT, COMP, KP>(c.device);
+  if (c.o.max_ctas > 0 && (long long)c.o.max_ctas * kWarps < W) W = (long long)c.o.max_ctas * kWarps;
+  if (W > units) W = units;
+  if (W < 1) W = 1;
+  return launch_ranges<VT, COMP, KP>(c, rw, (units + W - 1) / W * kTileNz);
+}
+
+// The even split over `threads` threads, a range per 32 of them.
+template <typename VT, bool COMP>
+el_status launch_shares(const SpmvCall& c, long long threads) {
+  const long long share = (c.A.rows + c.A.nnz + threads - 1) / threads;
+  return launch_ranges<VT, COMP, kPer>(c, 1, 32 * (share > 0 ? share : 1));
 }
 
 template <typename VT, bool COMP>
