@@ -3,7 +3,7 @@
 // Same split as spmv_merge_path_nz.cuh (equal merge ranges at diagonals
 // g * range_items, the reference's search [include/loops/schedule/
 // merge_path_flat.hxx:108-138, util/search.hxx:34-60]), but a range is a
-// CTA's: with at most one CTA per SM the time is a chain of memory round
+// CTA's: with everything resident at once the time is a chain of memory round
 // trips, so the CTA makes few of them -- offsets (all of them when there are
 // few rows, while the ticket is on its way), columns and values, x -- puts
 // the products in shared memory and sums rows from there, L lanes per row by
@@ -199,17 +199,19 @@ __global__ void __launch_bounds__(kSmTPB) merge_path_small_kernel(const Args a) 
   }
 }
 
-// One range of 2048 items per SM at most, and no option that shapes the warp
-// walk.  Passes after each other on the GB300, this kernel / the warp walk:
-// 6,000 nonzeros 6.2 / 10.3 us, 60,000 8.2 / 12.3, 150,000 10.2 / 12.2, 300,000
-// 12.3 / 12.4 (log-normal rows, mean 12; from there on the walk's 24 warps per
-// SM hide more than the shorter chain saves: 600,000 with ranges of 4096 15.4 /
-// 15.4, mean 35 16.4 / 12.4).
+// Four ranges of 2048 items per SM at most (five CTAs are resident), and no
+// option that shapes the warp walk.  Passes after each other on the GB300, this
+// kernel / the warp walk, log-normal rows of 13: 20,000 nonzeros 8.2 / 10.5 us,
+// 60,000 8.2 / 12.3, 200,000 10.3 / 12.4, 300,000 10.3 / 12.4, 500,000 12.3 /
+// 14.4, 800,000 14.4 / 16.4, 1.2M 16.5 / 18.6, 1.6M 18.5 / 18.6, 4M 39 / 29
+// (from there on the walk's 24 warps per SM hide more than the shorter chain
+// saves).
+constexpr int kSmCtasPerSm = 4;
 template <typename VT>
 bool small_fits(const SpmvCall& c) {
   if (c.o.max_ctas > 0 || c.o.nz_per_lane != 0) return false;
   const long long total = (long long)row_weight(c) * c.A.rows + c.A.nnz;
-  return total <= (long long)device_info(c.device).sm_count * kSmItems;
+  return total <= (long long)device_info(c.device).sm_count * kSmCtasPerSm * kSmItems;
 }
 
 template <typename VT>
@@ -217,9 +219,11 @@ el_status launch_small(const SpmvCall& c) {
   Args a;
   a.rw = row_weight(c);
   const long long total = (long long)a.rw * c.A.rows + c.A.nnz;
-  const long long sms = device_info(c.device).sm_count;
-  // whole 256-item units, as the warp ranges
-  const long long units = (total + kTileNz - 1) / kTileNz, upr = (units + sms - 1) / sms;
+  // whole 256-item units, as the warp ranges; four CTAs per SM cover each
+  // other's round trips (300,000 nonzeros: 12.3 us in ranges of 2048, 10.3 of
+  // 1024; 1.2M: 16.5 of 2048, 20.3 of 1024, two waves)
+  const long long ctas = (long long)device_info(c.device).sm_count * kSmCtasPerSm;
+  const long long units = (total + kTileNz - 1) / kTileNz, upr = (units + ctas - 1) / ctas;
   a.rows = c.A.rows;
   a.cols = c.A.cols;
   a.nnz = c.A.nnz;

@@ -1,5 +1,5 @@
 """merge_path on small matrices, by both of its kernels: a CTA per range (the
-default up to 2048 merge items per SM) and the warp walk (nz_per_lane=8 asks
+default up to 8192 merge items per SM) and the warp walk (nz_per_lane=8 asks
 for it at any size), at the sizes where the first can go wrong: one row, one
 nonzero, ranges of one unit (256 items), more rows than the offsets it keeps
 (4096), rows that are multiplied again from their start (up to 1024 nonzeros
@@ -35,13 +35,15 @@ def case(name, rng):
         return random_csr(rng, 40, 150_000, 5, long_rows=[(0, 9000), (3, 120_000), (39, 30_000)])
     if name == "empty":
         return random_csr(rng, 3000, 50, 0)
-    if name == "last_small":  # just under 2048 items per SM (152 SMs), weight 2
+    if name == "mid":
         return random_csr(rng, 20_000, 5000, 26)
-    return random_csr(rng, 30_000, 5000, 26)  # just over: the warp walk
+    if name == "last_small":  # just under 4 x 2048 items per SM (152 SMs), weight 2
+        return random_csr(rng, 20_000, 5000, 116)
+    return random_csr(rng, 21_500, 5000, 118)  # just over: the warp walk
 
 
 NAMES = ["one", "one_row", "unit", "rows_4096", "rows_4097", "many_rows", "again", "long",
-         "empty", "last_small", "first_walk"]
+         "empty", "mid", "last_small", "first_walk"]
 
 
 @pytest.mark.parametrize("dtype", ["f32", "bf16", "f16"])
