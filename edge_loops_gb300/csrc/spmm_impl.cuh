@@ -33,6 +33,7 @@ constexpr int kWarps = 4;       // per CTA
 constexpr int kTPB = 32 * kWarps;
 constexpr int kBlock = 4096;    // merge items of a range worked on at a time
 constexpr int kMaxNz = 2 * kBlock;  // nonzeros of a block, at most
+constexpr int kFold = 32;           // steps (a power of two)
 // Merge items per row end: a row end costs the walk about two nonzeros (its
 // test, store and new sum).
 constexpr int kRowItems = 2;
@@ -153,6 +154,7 @@ struct Smem {  // per warp
   unsigned rowm[kBlock / 32 + 4];  // bit i: row i of the block ends by such a bit
   float open[ORDERED ? 1 : NG][ORDERED ? 1 : L::kCols];  // a piece's open row
   float pend[ORDERED ? 1 : NG][ORDERED ? 1 : L::kCols];  // its part of the row it began inside
+  float fold[ORDERED ? 1 : L::P][32];  // the lanes' earlier sums of a long row
   int first[NG];     // a piece's first row
   int closed[NG];    // it closed a row
   int has_pend[NG];  // that first row began before the piece
@@ -383,6 +385,18 @@ struct Walk {
 #pragma unroll
     for (int k = 0; k < P; ++k) acc[k] = 0.f;
     bool has_pend = false;
+    // a long row's sum is put aside every kFold steps without a row end: short
+    // chains of additions, for the rounding error
+    bool folded = false;
+    auto unfold = [&]() {
+      if constexpr (!ORDERED) {
+        if (folded) {
+#pragma unroll
+          for (int k = 0; k < P; ++k) acc[k] = __fadd_rn(M.fold[k][lane], acc[k]);
+          folded = false;
+        }
+      }
+    };
     float* crow = a.C + (long long)x * a.ldc + L::column(sl, 0);
     float scn = scale && !lone ? __ldg(scale + min(x + sl, (int)a.rows - 1)) : 1.f;
     unsigned ends = step_ends(y);
@@ -440,10 +454,21 @@ struct Walk {
       if (!__any_sync(kFullMask, ends != 0)) {
 #pragma unroll
         for (int j = 0; j < U; ++j) add(v[j], b[j], acc);
+        if constexpr (!ORDERED) {
+          if ((i & (kFold - 1)) == kFold - 1) {
+#pragma unroll
+            for (int k = 0; k < P; ++k) {
+              M.fold[k][lane] = folded ? __fadd_rn(M.fold[k][lane], acc[k]) : acc[k];
+              acc[k] = 0.f;
+            }
+            folded = true;
+          }
+        }
       } else {
-        // the first row of a piece may be another's too, and a window of
-        // rows or scales may not reach the last end: those go one by one
-        bool each = ends != 0 && began;
+        // the first row of a piece may be another's too, a long row has sums
+        // put aside, and a window of rows or scales may not reach the last
+        // end: those go one by one
+        bool each = ends != 0 && (began || folded);
         unsigned rw = 0u;
         if (!dense) {
           rw = bits_at(M.rowm, min(x - rs, nrows));
@@ -476,6 +501,7 @@ struct Walk {
             }
             add(M.val[slot][grp * G + j], bj, acc);
             if ((ends >> j) & 1u) {
+              unfold();
               if (began) {
                 if constexpr (!ORDERED) {
 #pragma unroll
@@ -502,6 +528,7 @@ struct Walk {
       y = min(y + U, ye);
       ends = step_ends(y);
     }
+    unfold();
     if (lone && grp == 0) store(crow, acc, scale ? __ldg(scale + rs) : 1.f);
     __syncwarp();
     if constexpr (!ORDERED) {
