@@ -431,7 +431,7 @@ el_status el_batch_plan_create(const el_batch_item* items, int32_t count,
       dtype == EL_F32 ? (const void*)batch::batched_spmv_kernel<float>
                       : dtype == EL_BF16 ? (const void*)batch::batched_spmv_kernel<__nv_bfloat16>
                                          : (const void*)batch::batched_spmv_kernel<__half>,
-      256, 0);
+      256, 0, true);
   long long grid = (long long)std::max(per_sm, 1) * device_info(p->device).sm_count;
   if (o.max_ctas > 0) grid = std::min<long long>(grid, o.max_ctas);
   grid = std::min<long long>(grid, std::max(p->n_items, 1LL));

@@ -72,7 +72,7 @@ const DeviceInfo& device_info(int device) {
   return g_dev_info.emplace(device, d).first->second;
 }
 
-int resident_ctas_per_sm(const void* kernel, int threads, size_t smem) {
+int resident_ctas_per_sm(const void* kernel, int threads, size_t smem, bool prefer_l1) {
   int dev = 0;
   cudaGetDevice(&dev);
   const long long key2 = ((long long)dev << 48) ^ ((long long)threads << 32) ^ (long long)smem;
@@ -85,6 +85,15 @@ int resident_ctas_per_sm(const void* kernel, int threads, size_t smem) {
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, threads, smem) !=
       cudaSuccess)
     n = 0;
+  cudaFuncAttributes at;
+  if (prefer_l1 && n > 0 && cudaFuncGetAttributes(&at, kernel) == cudaSuccess) {
+    // no more shared memory than those CTAs use (1 KB each is the system's),
+    // in percent of the 228 KB an SM can carve out
+    const size_t need = (size_t)n * (at.sharedSizeBytes + smem + 1024);
+    const int percent = (int)((need * 100 + 228 * 1024 - 1) / (228 * 1024));
+    cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                         percent < 100 ? percent : 100);
+  }
   std::lock_guard<std::mutex> lk(g_mu);
   g_occupancy[{kernel, key2}] = n;
   return n;

@@ -27,8 +27,12 @@ struct DeviceInfo {
 const DeviceInfo& device_info(int device);
 
 // Resident CTAs per SM for a kernel at a block size and dynamic smem size
-// (cached per kernel and configuration).
-int resident_ctas_per_sm(const void* kernel, int threads, size_t smem);
+// (cached per kernel and configuration).  prefer_l1 leaves the kernel the
+// largest L1 beside that many CTAs: the driver's own choice for the merge-path
+// walk (3 x 20 KB) is a 135 KB carve-out, which halves the L1 that x is
+// gathered through (batched BF16 plan 310 -> 284 us with 64 KB, power-law
+// matrix 78.5 -> 76.4, 96^3 stencil by group_mapped 60 -> 58).
+int resident_ctas_per_sm(const void* kernel, int threads, size_t smem, bool prefer_l1 = false);
 
 // Everything a SpMV launcher needs; pointers already validated.
 struct SpmvCall {

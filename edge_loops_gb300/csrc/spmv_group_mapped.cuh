@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(kTPB, 3)
 
 template <typename VT, bool COMP>
 el_status launch_group_mapped_rows(const SpmvCall& c, int group_rows) {
-  const int per_sm = resident_ctas_per_sm((const void*)group_mapped_kernel<VT, COMP>, kTPB, 0);
+  const int per_sm = resident_ctas_per_sm((const void*)group_mapped_kernel<VT, COMP>, kTPB, 0, true);
   const long long ctas = (long long)(per_sm > 0 ? per_sm : 1) * device_info(c.device).sm_count;
   Src m{c.A.offsets, c.A.indices, c.A.values, c.A.row_scale, c.x, c.y,
         (int)c.A.rows, (unsigned)c.A.cols, (int)c.A.nnz, 0, 0};

@@ -667,7 +667,7 @@ inline int row_weight(const SpmvCall& c) {
 template <typename VT, bool COMP, int KP = kPer>
 int resident_warps(int device) {
   const int per_sm =
-      resident_ctas_per_sm((const void*)merge_path_nz_kernel<VT, COMP, KP>, kTPB, 0);
+      resident_ctas_per_sm((const void*)merge_path_nz_kernel<VT, COMP, KP>, kTPB, 0, true);
   return (per_sm > 0 ? per_sm : 1) * kWarps * device_info(device).sm_count;
 }
 
