@@ -34,6 +34,12 @@ constexpr int kTPB = 32 * kWarps;
 constexpr int kBlock = 4096;    // merge items of a range worked on at a time
 constexpr int kMaxNz = 2 * kBlock;  // nonzeros of a block, at most
 constexpr int kFold = 32;           // steps (a power of two)
+// ORDERED: longer rows are walked by the whole warp, which has 32 / G times the
+// B rows in flight (a group alone takes 0.45 us per 8 nonzeros); shorter ones
+// cost more to set apart than that saves.  Threshold none / 512 / 256 / 128:
+// 3,000 log-normal rows of 20, n = 9, 74 / 44 / 35 / 31 us; 60,000 of them,
+// n = 64, 93 / 70 / 64 / 64; 200,003 of 10, n = 24, 58 / 58 / 58 / 70.
+constexpr int kLongRow = 256;
 // Merge items per row end: a row end costs the walk about two nonzeros (its
 // test, store and new sum).
 constexpr int kRowItems = 2;
@@ -169,6 +175,8 @@ template <typename L, bool ORDERED>
 struct Walk {
   using Sm = Smem<L, ORDERED>;
   static constexpr int G = L::G, U = L::U, NG = 32 / G, P = L::P, V = L::V, K = L::K;
+  // (a block closes at most kBlock nonzeros beside its first row's)
+  static constexpr int kLong = NG > 1 ? kLongRow : kMaxNz - kBlock;
   const Args& a;
   Sm& M;
   const int lane, sl, grp;
@@ -240,116 +248,175 @@ struct Walk {
     }
   }
 
+  // One long row, nonzeros [b, e) in order, by the whole warp: the groups read
+  // the B rows of NG U nonzeros at once and add their products in turn, each
+  // group to the sum the one before it hands on.
+  __device__ __forceinline__ void long_row(int row, int b, int e) {
+    float acc[P];
+#pragma unroll
+    for (int k = 0; k < P; ++k) acc[k] = 0.f;
+    Nz nz;
+    const int mine = grp * U + sl;  // this lane's nonzero of a step (sl < U)
+    nz.load(a, sl < U && b + mine < e, b + mine);
+    int slot = 0;
+#pragma unroll 1
+    for (int y = b; y < e; y += NG * U, slot ^= 1) {
+      const bool ok = (unsigned)nz.c < (unsigned long long)a.cols;
+      M.idx[slot][lane] = ok ? nz.c : -1;
+      M.val[slot][lane] = ok ? nz.value(a) : 0.f;
+      bad_col |= sl < U && y + mine < e && !ok;
+      const int next = y + NG * U + mine;
+      nz.load(a, sl < U && next < e, next);
+      __syncwarp();
+      BVec<L> bv[U][K];
+#pragma unroll
+      for (int j = 0; j < U; ++j) {
+        const int c = M.idx[slot][grp * G + j];
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          bv[j][k].zero();
+          if (c >= 0) bv[j][k].load(my_B[k] + (unsigned long long)(unsigned)c * a.ldb);
+        }
+      }
+#pragma unroll 1
+      for (int g = 0; g < NG; ++g) {
+        if (grp == g) {  // a nonzero past the end adds 0 * 0 to a sum that is never -0
+#pragma unroll
+          for (int j = 0; j < U; ++j) add(M.val[slot][grp * G + j], bv[j], acc);
+        }
+        __syncwarp();
+        if (NG > 1) {
+#pragma unroll
+          for (int k = 0; k < P; ++k) acc[k] = __shfl_sync(kFullMask, acc[k], g * G + sl);
+        }
+      }
+    }
+    if (grp == 0)
+      store(a.C + (long long)row * a.ldc + L::column(sl, 0), acc,
+            a.row_scale ? __ldg(a.row_scale + row) : 1.f);
+    __syncwarp();
+  }
+
   // One block: rows [rs, re) and nonzeros [ns, ne), the rows' ends among
   // them.  `inside`: row rs began before nonzero ns.  z_out: row rs ends here
-  // without a nonzero.  lone: one row, too long for the bit array, by group 0.
+  // without a nonzero.  ORDERED: stops before the first long row; returns the
+  // row it stopped at.
   // Leaves every piece's open row in M.open, with M.first, closed, has_pend.
-  __device__ __forceinline__ void block(const int rs, const int re, const int ns, const int ne,
-                                        const bool inside, const bool lone, bool& z_out) {
+  __device__ __forceinline__ int block(const int rs, int re, const int ns, int ne,
+                                       const bool inside, bool& z_out) {
     const float* const scale = a.row_scale;
-    const int len = ne - ns, nrows = re - rs;
+    int len = ne - ns, nrows = re - rs;
     // pieces: equal shares of the nonzeros in whole steps (ORDERED: moved to
     // row starts below)
-    const int per = lone ? len : (len + NG * U - 1) / (NG * U) * U;
+    auto share = [&]() { return (len + NG * U - 1) / (NG * U) * U; };
+    int per = share();
     const long long y0 = ns + (long long)per * grp;
     int y = y0 < ne ? (int)y0 : ne;
     int ye = y0 + per < ne ? (int)(y0 + per) : ne;
     Nz nz;
-    if (!ORDERED || lone) nz.load(a, sl < U && y + sl < ye, y + sl);
+    if (!ORDERED) nz.load(a, sl < U && y + sl < ye, y + sl);
 
     // the row ends as bits; empty rows are written here
     bool dense = true;
     z_out = false;
-    if (!lone) {
-      for (int i = lane; i < (len >> 5) + 2; i += 32) M.ends[i] = 0u;
-      for (int i = lane; i < (nrows >> 5) + 2; i += 32) M.rowm[i] = 0u;
-      __syncwarp();
-      for (int i0 = 0; i0 < nrows; i0 += 128) {
-        int s4[4], e4[4];
+    for (int i = lane; i < (min(len, kMaxNz) >> 5) + 2; i += 32) M.ends[i] = 0u;
+    for (int i = lane; i < (nrows >> 5) + 2; i += 32) M.rowm[i] = 0u;
+    __syncwarp();
+    for (int i0 = 0; i0 < nrows; i0 += 128) {
+      int s4[4], e4[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int i = i0 + 32 * u + lane;
-          s4[u] = i < nrows ? __ldg(a.offsets + rs + i) : 0;
-          e4[u] = i < nrows ? __ldg(a.offsets + rs + i + 1) : 0;
+      for (int u = 0; u < 4; ++u) {
+        const int i = i0 + 32 * u + lane;
+        s4[u] = i < nrows ? __ldg(a.offsets + rs + i) : 0;
+        e4[u] = i < nrows ? __ldg(a.offsets + rs + i + 1) : 0;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (i0 + 32 * u >= nrows) break;
+        const int i = i0 + 32 * u + lane, s = s4[u], e = e4[u];
+        if constexpr (ORDERED) {
+          const unsigned lm = __ballot_sync(kFullMask, i < nrows && e - s > kLong);
+          if (lm) {  // the block ends before this row
+            const int q = __ffs(lm) - 1;
+            nrows = i0 + 32 * u + q;
+            ne = min(max(__shfl_sync(kFullMask, s, q), ns), ne);
+          }
         }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          if (i0 + 32 * u >= nrows) break;
-          const int i = i0 + 32 * u + lane, s = s4[u], e = e4[u];
-          const bool empty = i < nrows && s == e;
-          const bool z = !ORDERED && i == 0 && inside && e == ns;
-          const bool bit = i < nrows && !empty && !z && e > ns && e <= ne;
-          if (bit) {
-            const unsigned m = 1u << ((e - ns - 1) & 31);
-            bad_off |= (atomicOr(&M.ends[(e - ns - 1) >> 5], m) & m) != 0;
-          }
-          bad_off |= i < nrows && !empty && !z && (!bit || e < s || (ORDERED && s < ns));
-          z_out |= __any_sync(kFullMask, z);
-          const unsigned rb = __ballot_sync(kFullMask, bit);
-          if (lane == 0) M.rowm[i >> 5] = rb;
-          dense = dense && rb == __ballot_sync(kFullMask, i < nrows);
-          for (unsigned em = __ballot_sync(kFullMask, empty); em; em &= em - 1) {
-            const long long row = rs + i0 + 32 * u + __ffs(em) - 1;
-            const float zero = scale ? 0.f * __ldg(scale + row) : 0.f;
-            for (int c = lane; c < a.n; c += 32) __stcs(a.C + row * a.ldc + c, zero);
-          }
+        const bool empty = i < nrows && s == e;
+        const bool z = !ORDERED && i == 0 && inside && e == ns;
+        const bool bit = i < nrows && !empty && !z && e > ns && e <= ne && e - ns <= kMaxNz;
+        if (bit) {
+          const unsigned m = 1u << ((e - ns - 1) & 31);
+          bad_off |= (atomicOr(&M.ends[(e - ns - 1) >> 5], m) & m) != 0;
+        }
+        bad_off |= i < nrows && !empty && !z && (!bit || e < s || (ORDERED && s < ns));
+        z_out |= __any_sync(kFullMask, z);
+        const unsigned rb = __ballot_sync(kFullMask, bit);
+        if (lane == 0) M.rowm[i >> 5] = rb;
+        dense = dense && rb == __ballot_sync(kFullMask, i < nrows);
+        for (unsigned em = __ballot_sync(kFullMask, empty); em; em &= em - 1) {
+          const long long row = rs + i0 + 32 * u + __ffs(em) - 1;
+          const float zero = scale ? 0.f * __ldg(scale + row) : 0.f;
+          for (int c = lane; c < a.n; c += 32) __stcs(a.C + row * a.ldc + c, zero);
         }
       }
-      __syncwarp();
+    }
+    __syncwarp();
+    if (ORDERED) {
+      re = rs + nrows;
+      len = ne - ns;
+      if (len > kMaxNz) bad_off = true;  // malformed offsets
+      if (nrows == 0 || len > kMaxNz) return re;
+      per = share();
     }
 
     // the row each piece starts in
     int x = rs;
     bool began = grp == 0 && inside;
-    if (!lone) {
-      int before = 0;  // the row ends before this group's piece
+    int before = 0;  // the row ends before this group's piece
 #pragma unroll
-      for (int p = 1; p < NG; ++p) {
-        const int q = min(per * p, len);
-        int c = 0;
-        for (int i = lane; i <= q >> 5; i += 32) {
-          unsigned m = M.ends[i];
-          if (i == q >> 5) m &= (1u << (q & 31)) - 1u;
-          c += __popc(m);
+    for (int p = 1; p < NG; ++p) {
+      const int q = min(per * p, len);
+      int c = 0;
+      for (int i = lane; i <= q >> 5; i += 32) {
+        unsigned m = M.ends[i];
+        if (i == q >> 5) m &= (1u << (q & 31)) - 1u;
+        c += __popc(m);
+      }
+      c = __reduce_add_sync(kFullMask, c);
+      if (p == grp) before = c;
+    }
+    if (dense) {
+      x = rs + before;
+    } else {
+      // the `before`-th set bit of rowm (re when there is none)
+      int skip = before, at = nrows;
+      for (int i = 0; i <= nrows >> 5; ++i) {
+        const unsigned m = M.rowm[i];
+        const int c = __popc(m);
+        if (skip >= 0 && skip < c) {
+          unsigned t = m;
+          for (int k = 0; k < skip; ++k) t &= t - 1;
+          at = 32 * i + __ffs(t) - 1;
+          skip = -1;
+        } else if (skip >= 0) {
+          skip -= c;
         }
-        c = __reduce_add_sync(kFullMask, c);
-        if (p == grp) before = c;
       }
-      if (dense) {
-        x = rs + before;
-      } else {
-        // the `before`-th set bit of rowm (re when there is none)
-        int skip = before, at = nrows;
-        for (int i = 0; i <= nrows >> 5; ++i) {
-          const unsigned m = M.rowm[i];
-          const int c = __popc(m);
-          if (skip >= 0 && skip < c) {
-            unsigned t = m;
-            for (int k = 0; k < skip; ++k) t &= t - 1;
-            at = 32 * i + __ffs(t) - 1;
-            skip = -1;
-          } else if (skip >= 0) {
-            skip -= c;
-          }
-        }
-        x = rs + min(at, nrows);
-      }
-      if (ORDERED) {
-        // whole rows: from row x's start to the next piece's row's
-        y = x < re ? min(max(__ldg(a.offsets + x), ns), ne) : ne;
-        ye = __shfl_down_sync(kFullMask, y, G);
-        if (grp == NG - 1) ye = ne;
-        ye = max(y, ye);
-        nz.load(a, sl < U && y + sl < ye, y + sl);
-      } else if (y > ns) {
-        const int q = y - ns - 1;
-        began = !((M.ends[q >> 5] >> (q & 31)) & 1u);
-      } else {
-        began = inside && !z_out;
-      }
-    } else if (grp > 0) {
-      y = ye = ne;
-      x = re;
+      x = rs + min(at, nrows);
+    }
+    if (ORDERED) {
+      // whole rows: from row x's start to the next piece's row's
+      y = x < re ? min(max(__ldg(a.offsets + x), ns), ne) : ne;
+      ye = __shfl_down_sync(kFullMask, y, G);
+      if (grp == NG - 1) ye = ne;
+      ye = max(y, ye);
+      nz.load(a, sl < U && y + sl < ye, y + sl);
+    } else if (y > ns) {
+      const int q = y - ns - 1;
+      began = !((M.ends[q >> 5] >> (q & 31)) & 1u);
+    } else {
+      began = inside && !z_out;
     }
     const int x0 = x;
     int steps = (ye - y + U - 1) / U;
@@ -357,7 +424,7 @@ struct Walk {
     for (int d = G; d < 32; d <<= 1) steps = max(steps, __shfl_xor_sync(kFullMask, steps, d));
 
     auto step_ends = [&](int at) -> unsigned {  // the piece's row ends in [at, at + U)
-      if (lone || at >= ye) return 0u;
+      if (at >= ye) return 0u;
       const int q = at - ns;
       if (!ORDERED) {
         const unsigned b = reinterpret_cast<const unsigned char*>(M.ends)[q >> 3];
@@ -398,7 +465,7 @@ struct Walk {
       }
     };
     float* crow = a.C + (long long)x * a.ldc + L::column(sl, 0);
-    float scn = scale && !lone ? __ldg(scale + min(x + sl, (int)a.rows - 1)) : 1.f;
+    float scn = scale ? __ldg(scale + min(x + sl, (int)a.rows - 1)) : 1.f;
     unsigned ends = step_ends(y);
 #pragma unroll 1
     for (int i = 0; i < steps; ++i) {
@@ -529,7 +596,6 @@ struct Walk {
       ends = step_ends(y);
     }
     unfold();
-    if (lone && grp == 0) store(crow, acc, scale ? __ldg(scale + rs) : 1.f);
     __syncwarp();
     if constexpr (!ORDERED) {
       if (sl == 0) {
@@ -543,6 +609,7 @@ struct Walk {
         for (int t = 0; t < V; ++t) M.open[grp][L::column(sl, k) + t] = acc[V * k + t];
       __syncwarp();
     }
+    return re;
   }
 };
 
@@ -592,24 +659,20 @@ __global__ void __launch_bounds__(kTPB, kMinCtas) spmm_kernel(const Args a) {
       const int m = (int)a.nnz;
       ns = min(max(sa.start, 0), m);
       ne = min(max(sb.start, ns), m);
-      if (rs < re && ne - ns > kMaxNz) {  // the first of them is longer than a block
-        const int e = min(max(__ldg(a.offsets + rs + 1), ns), ne);
-        walk.block(rs, rs + 1, ns, e, false, true, z);
-        ++rs;
-        ns = e;
-        if (ne - ns > kMaxNz) {  // malformed offsets
-          walk.bad_off = true;
-          ne = ns;
-        }
+      while (rs < re) {  // runs of shorter rows, and each long row by itself
+        rs = walk.block(rs, re, ns, ne, false, z);
+        if (rs >= re) break;
+        const int b = min(max(__ldg(a.offsets + rs), ns), ne);
+        ns = min(max(__ldg(a.offsets + rs + 1), b), ne);
+        walk.long_row(rs++, b, ns);
       }
-      if (rs < re) walk.block(rs, re, ns, ne, false, false, z);
     } else {
       if (d == d0) {
         r0 = rs;
         n0 = ns;
         off_r0 = sa.start;
       }
-      walk.block(rs, re, ns, ne, ns > sa.start, false, z);
+      walk.block(rs, re, ns, ne, ns > sa.start, z);
       // stitch the rows that cross pieces, in piece order
       const bool need_lb = n0 > off_r0;
       if (z) {  // row rs ended at the block's first nonzero

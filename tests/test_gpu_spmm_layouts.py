@@ -120,6 +120,26 @@ def test_many_rows_and_mostly_empty_ones(cuda, oracle_mod, empty):
             assert np.all(np.abs(got - C64) <= k * U / (1 - k * U) * Ca)
 
 
+@pytest.mark.parametrize("n", [3, 8, 16, 24, 33, 64, 128])
+def test_rows_around_the_long_row_threshold(cuda, oracle_mod, n):
+    """Rows of 255 .. 258 nonzeros beside short and empty ones, first, last and
+    next to each other: the ordered schedules set the long ones apart."""
+    from edge_loops_gb300 import api
+    rng = np.random.default_rng(n)
+    long_rows = [(0, 257), (1, 256), (2, 258), (3, 257), (40, 255), (41, 0), (42, 600),
+                 (43, 0), (100, 4096), (101, 4000), (150, 4097), (151, 4000), (299, 300)]
+    off, idx, vals = random_csr(rng, rows=300, cols=6000, max_len=20, empty_frac=0.1,
+                                long_rows=long_rows)[:3]
+    B = rng.uniform(-1, 1, size=(6000, n)).astype(np.float32)
+    A = api.CSR.from_arrays(off, idx, vals, 6000, device=cuda)
+    exp = oracle_mod.spmm_f32(off, idx, vals, B)
+    for sched in ("thread_mapped", "group_mapped"):
+        C = torch.full((300, n), float("nan"), device=cuda)
+        api.spmm(A, torch.as_tensor(B, device=cuda), C, schedule=sched)
+        assert api.workspace_errors() == 0
+        np.testing.assert_array_equal(C.cpu().numpy(), exp)
+
+
 @pytest.mark.parametrize("sched", ["thread_mapped", "merge_path_flat"])
 def test_bad_columns_are_flagged_and_read_nothing(cuda, ragged, sched):
     """Columns outside [0, cols) contribute nothing, whatever B holds, and
