@@ -4,11 +4,12 @@
 
 namespace el {
 
-// Warp ranges of the merge-path SpMM: at most one per warp that can be
-// resident (2048 threads per SM), with a carry slot and a row vector of 128
-// floats each.
+// Warp ranges of the merge-path SpMM, at most: 48 per SM (24 are resident),
+// with a carry slot and a row vector of 128 floats each.  No more slots than a
+// new workspace has: one that grew would leave a graph captured before with
+// the memory it had.
 static long long spmm_mp_ranges(const SpmmCall& c) {
-  return (long long)device_info(c.device).sm_count * 64;
+  return (long long)device_info(c.device).sm_count * 48;
 }
 
 size_t spmm_scratch_bytes(const SpmmCall& c, int schedule) {

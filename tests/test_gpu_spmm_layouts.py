@@ -158,3 +158,23 @@ def test_bad_columns_are_flagged_and_read_nothing(cuda, ragged, sched):
         ref = api.spmm(api.CSR.from_arrays(off, idx, v0, 20_000, device=cuda), B, schedule=sched)
         assert api.workspace_errors() == 0
         assert torch.equal(C, ref)
+
+
+def test_keeps_a_captured_spmv(cuda, ragged):
+    """An SpMM takes no more carry slots than a new workspace has, so a graph
+    captured with the workspace before it still finds its memory there."""
+    from edge_loops_gb300 import api
+    off, idx, vals = ragged
+    A = api.CSR.from_arrays(off, idx, vals, 20_000, device=cuda)
+    x = torch.rand(20_000, device=cuda)
+    exp = api.spmv(A, x).cpu()
+    y = torch.full((700,), float("nan"), device=cuda)
+    ws = api.Workspace()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        api.spmv(A, x, y, workspace=ws)
+    C = api.spmm(A, torch.rand(20_000, 8, device=cuda), workspace=ws)
+    g.replay()
+    torch.cuda.synchronize()
+    assert ws.errors() == 0 and torch.equal(y.cpu(), exp) and bool(C.isfinite().all())
