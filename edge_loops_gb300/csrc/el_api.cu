@@ -35,7 +35,6 @@ std::map<std::pair<int, cudaStream_t>, el_workspace*> g_default_ws;
 std::map<int, DeviceInfo> g_dev_info;
 std::map<std::pair<const void*, long long>, int> g_occupancy;
 
-constexpr long long kInitialSlots = 8192;
 constexpr unsigned long long kDefaultWaitNs = 2000000000ull;  // 2 s
 }  // namespace
 

@@ -15,6 +15,9 @@ namespace el {
 // a tile's extent (at most a few thousand items) never leaves int32.
 constexpr long long kMergeLimit = (1LL << 31) - (1LL << 16);
 
+// Carry slots of a new workspace.
+constexpr long long kInitialSlots = 8192;
+
 // Records a failure for el_last_error_string() and returns `s`.
 el_status fail(el_status s, const char* fmt, ...);
 // EL_OK on cudaSuccess, else EL_ERR_CUDA with the CUDA error text.

@@ -146,7 +146,8 @@ struct SpmvImpl {
   static long long work_oriented_slots(const SpmvCall& c) {
     const long long m = c.o.compensated ? mpn::slots_needed<VT, true>(c)
                                         : mpn::slots_needed<VT, false>(c);
-    const long long n = (c.o.num_threads + 31) / 32;
+    const long long nt = c.o.num_threads > 0 ? c.o.num_threads : 0, t = mpn::share_threads(nt);
+    const long long n = (nt + t - 1) / t;
     return n > m ? n : m;
   }
   template <bool COMP>

@@ -1,5 +1,6 @@
 // spmv_merge_path_nz.cuh -- merge-path SpMV for sm_103a, nonzero-tiled warp
-// variant (the default).
+// variant: the default merge path but for small matrices
+// (spmv_merge_path_small.cuh), and work_oriented.
 //
 // The work split follows the reference's merge_path_flat schedule at the
 // level of warp ranges [include/loops/schedule/merge_path_flat.hxx:108-138,
@@ -746,11 +747,19 @@ el_status launch_kp(const SpmvCall& c) {
   return launch_ranges<VT, COMP, KP>(c, rw, (units + W - 1) / W * kTileNz);
 }
 
-// The even split over `threads` threads, a range per 32 of them.
+// The even split over `threads` threads, a range per 32 of them, or per 64 or
+// 128 where 32 would need more carry slots than a new workspace has (a
+// workspace that grew would leave a graph captured before with the memory it
+// had).
+inline long long share_threads(long long threads) {
+  long long t = 32;
+  while (t < 128 && threads > kInitialSlots * t) t *= 2;
+  return t;
+}
 template <typename VT, bool COMP>
 el_status launch_shares(const SpmvCall& c, long long threads) {
   const long long share = (c.A.rows + c.A.nnz + threads - 1) / threads;
-  return launch_ranges<VT, COMP, kPer>(c, 1, 32 * (share > 0 ? share : 1));
+  return launch_ranges<VT, COMP, kPer>(c, 1, share_threads(threads) * (share > 0 ? share : 1));
 }
 
 template <typename VT, bool COMP>

@@ -73,6 +73,29 @@ def test_16bit_values_with_scales(cuda, oracle_mod, name, sched, dtype):
     assert np.all(np.abs(y.cpu().numpy() - y64) <= order_free_bound(off, yabs, extra=3))
 
 
+@pytest.mark.parametrize("num_threads", [8192 * 32, 8192 * 32 + 128, 8192 * 64, 8192 * 128])
+def test_many_threads_under_capture(cuda, oracle_mod, num_threads):
+    """A new workspace has the carry slots of every thread count up to
+    8192 x 128: nothing is allocated under capture."""
+    from edge_loops_gb300 import api
+    off, idx, vals, x = case("more")
+    A = api.CSR.from_arrays(off, idx, vals, len(x), device=cuda)
+    xt = torch.as_tensor(x, device=cuda)
+    y = torch.full((A.rows,), float("nan"), device=cuda)
+    api.spmv(A, xt, y, schedule="work_oriented", workspace=api.Workspace())
+    y.fill_(float("nan"))
+    ws = api.Workspace()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        api.spmv(A, xt, y, schedule="work_oriented", workspace=ws, num_threads=num_threads)
+    g.replay()
+    torch.cuda.synchronize()
+    assert ws.errors() == 0
+    y64, yabs = oracle_mod.spmv_f64(off, idx, vals, x)
+    assert np.all(np.abs(y.cpu().numpy() - y64) <= order_free_bound(off, yabs))
+
+
 def test_num_threads_is_checked(cuda):
     from edge_loops_gb300 import _lib, api
     off, idx, vals, x = case("rows33")
