@@ -1046,11 +1046,12 @@ def run_csr_build(args):
         "data": "synthetic (the power-law SpMV matrix's entries in random order)",
         "config": {"workload": "COO of the 2^20 x 2^20 power-law matrix (seed 1), shuffled",
                    "nnz": nnz, "rows": rows, "bytes_per_step": nbytes,
-                   "includes": "range check (one host sync), radix sort, gather, offsets"},
+                   "includes": "row counts, prefix sums, move to windows, range check "
+                               "(one host sync), window sort"},
         "check": {"equal_to_numpy_construction": ok},
         "cpu_baseline": {"value": round(nbytes / cpu_s / 1e9, 3), "unit": "GB/s", "cores": 1,
                          "kind": "port", "sample": "numpy stable lexsort + searchsorted, once"},
-        "gpu_launches": 3 * args.steps,  # this library's kernels; the radix sort is CUB's
+        "gpu_launches": 6 * args.steps,
     }
 
 

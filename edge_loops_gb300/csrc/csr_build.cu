@@ -709,7 +709,8 @@ extern "C" el_status el_csr_from_coo(el_workspace* ws, const el_coo* coo, int32_
   // atomics (entries / 4096 x windows) few: 2M entries 197 us by windows of
   // 2048, 3M 193 us by windows of 8192.
   bool done = false;
-  if (nnz >= Win<11>::W && coo->rows <= 2 * nnz + (1 << 20) && nnz <= (long long)kMaxWindows * Win<13>::W) {
+  if (nnz >= Win<11>::W && coo->rows <= 2 * nnz + (1 << 20) &&
+      nnz <= (long long)kMaxWindows * Win<13>::W) {
     st = nnz <= kSmallNnz ? window_sort<11>(w, coo, offsets, indices, values, s, sms, &done)
                           : window_sort<13>(w, coo, offsets, indices, values, s, sms, &done);
     if (st != EL_OK || done) return st;

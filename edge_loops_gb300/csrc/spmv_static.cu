@@ -1,10 +1,10 @@
 // spmv_static.cu -- el_spmv_static_scratch: the merge-path SpMV (the
-// default nonzero-tiled warp kernel) with its scratch in a fixed device
+// nonzero-tiled warp kernel) with its scratch in a fixed device
 // array instead of a workspace, for callers that must not allocate device
 // memory (see the declaration in include/edge_loops.h).
 //
-// The scratch is g_static_scratch: a WsHeader (range ticket, finished-warp
-// counter, error flags, launch epoch) followed by EL_STATIC_MAX_RANGES
+// The scratch is g_static_scratch: a WsHeader (range ticket, launch
+// epoch, error flags) followed by EL_STATIC_MAX_RANGES
 // carry slots.  It is a module-scope __device__ array, so every GPU that
 // loads this library holds it (64 KiB + 64 B) until the process exits, and
 // every call on a device shares it.  Host code may not use the array's name

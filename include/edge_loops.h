@@ -149,10 +149,9 @@ typedef struct el_spmv_opts {
                                 threads_per_block (block_mapped) */
   int64_t num_threads;       /* work_oriented: threads of the even split,
                                 a multiple of 128 (the reference uses
-                                2 x SMs x 128); 0 = the resident blocks'
-                                threads, or one per 256 merge items when
-                                that is more (at most 16 x SMs x 128), and
-                                none with fewer than 32 merge items */
+                                2 x SMs x 128); 0 = 32 per resident warp.
+                                A warp walks the shares of 32 threads
+                                together */
   int32_t compensated;       /* 1: Neumaier / two-sum compensated FP32 sums */
   int32_t max_ctas;          /* cap on persistent grids (0 = resident) */
   int32_t wait_limit_us;     /* bound on every device-side wait (0 = 2 s) */
@@ -195,8 +194,10 @@ typedef struct el_spmv_opts {
                                 tile walk, 8 (tiles of 256) or 16 (tiles of 512);
                                 0 = 16 for 16-bit values on matrices with at
                                 least 24 nonzeros per row on average and 2^20
-                                nonzeros in all, else 8.  Same results within
-                                the FP32 bound (the summation order changes) */
+                                nonzeros in all, else 8, and a CTA per range
+                                instead of the walk for small matrices.  Same
+                                results within the FP32 bound (the summation
+                                order changes) */
   int32_t reserved[3];
 } el_spmv_opts;
 
