@@ -92,55 +92,72 @@ size_t round256(size_t b) { return (b + 255) & ~(size_t)255; }
 // -------------------------------------------------------------- window sort
 // Row lengths by atomics, and the range check.  Atomics on one address run
 // one after the other (about 1.8 ns each), so a long row would set the time
-// (100,000 entries: 180 us); `copies` (a power of two) counters per row, one
-// per warp in turn, cut that chain.  SMALL: few rows, counted in shared memory
-// first.
+// (100,000 entries: 180 us).  Each CTA counts the rows that come to it first
+// in a table in shared memory, a slot per row, and the rest in global memory:
+// a row that comes often soon has a slot.  15.4M power-law entries of 2^20 rows
+// 87 us, of which the global atomics take 77 (eight counters per row without a
+// table: 137, and 26 more in the sums).  SMALL: few rows, all counted in shared
+// memory.
 constexpr int kSmallRows = 8192;
+constexpr int kCountThreads = 1024;
+constexpr int kTableLog = 12;
 template <bool SMALL>
-__global__ void count_rows_kernel(const int32_t* __restrict__ ri, const int32_t* __restrict__ ci,
-                                  long long nnz, long long rows, long long cols,
-                                  unsigned* __restrict__ len, int copies,
-                                  unsigned* __restrict__ flags) {
-  __shared__ unsigned s_len[SMALL ? kSmallRows : 1];
-  if (SMALL) {
-    for (int i = threadIdx.x; i < (int)rows; i += blockDim.x) s_len[i] = 0u;
-    __syncthreads();
-  } else {
-    len += (long long)((blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) & (copies - 1)) *
-           (rows + 1);
+__global__ void __launch_bounds__(kCountThreads, 2)
+    count_rows_kernel(const int32_t* __restrict__ ri, const int32_t* __restrict__ ci, int nnz,
+                      unsigned rows, unsigned cols, unsigned* __restrict__ len,
+                      unsigned* __restrict__ flags) {
+  constexpr int kSlots = SMALL ? kSmallRows : 1 << kTableLog;
+  constexpr unsigned kEmpty = 0xffffffffu;
+  __shared__ unsigned s_len[kSlots], s_row[SMALL ? 1 : kSlots];
+  for (int i = threadIdx.x; i < (SMALL ? (int)rows : kSlots); i += kCountThreads) {
+    s_len[i] = 0u;
+    if (!SMALL) s_row[i] = kEmpty;
   }
-  const long long step = (long long)gridDim.x * blockDim.x;
+  __syncthreads();
+  auto add = [&](unsigned r, unsigned v) {
+    if (SMALL) {
+      atomicAdd(s_len + r, v);
+      return;
+    }
+    const unsigned h = r * 0x9e3779b1u >> (32 - kTableLog);
+    unsigned own = *const_cast<volatile unsigned*>(s_row + h);
+    if (own == kEmpty) {
+      own = atomicCAS(s_row + h, kEmpty, r);
+      if (own == kEmpty) own = r;
+    }
+    if (own == r)
+      atomicAdd(s_len + h, v);
+    else
+      atomicAdd(len + r, v);
+  };
+  const int step = gridDim.x * kCountThreads;  // 4 steps past nnz (at most 2^27) fit an int
   // warp-uniform: k0 - lane counts
-  for (long long k0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; k0 - (threadIdx.x & 31) < nnz;
+  for (int k0 = blockIdx.x * kCountThreads + threadIdx.x; k0 - (int)(threadIdx.x & 31) < nnz;
        k0 += 4 * step) {
     int r[4], c[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const long long k = k0 + u * step;
+      const int k = k0 + u * step;
       r[u] = k < nnz ? __ldcs(ri + k) : -1;
       c[u] = k < nnz ? __ldcs(ci + k) : -1;
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const bool ok = (unsigned long long)(unsigned)r[u] < (unsigned long long)rows &&
-                      (unsigned long long)(unsigned)c[u] < (unsigned long long)cols;
+      const bool ok = (unsigned)r[u] < rows && (unsigned)c[u] < cols;
       if (!ok && k0 + u * step < nnz) atomicOr(flags, 1u);
-      unsigned* const p = SMALL ? s_len : len;
       // entries in row order: one atomic for a warp in one row
       const int r0 = __shfl_sync(kFullMask, r[u], 0);
       const bool same = ok && r[u] == r0;
       if (__all_sync(kFullMask, same)) {
-        if ((threadIdx.x & 31) == 0) atomicAdd(p + r0, 32u);
+        if ((threadIdx.x & 31) == 0) add(r0, 32u);
       } else if (ok) {
-        atomicAdd(p + r[u], 1u);
+        add(r[u], 1u);
       }
     }
   }
-  if (SMALL) {
-    __syncthreads();
-    for (int i = threadIdx.x; i < (int)rows; i += blockDim.x)
-      if (s_len[i]) atomicAdd(len + i, s_len[i]);
-  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < (SMALL ? (int)rows : kSlots); i += kCountThreads)
+    if (s_len[i]) atomicAdd(len + (SMALL ? (unsigned)i : s_row[i]), s_len[i]);
 }
 
 // Row starts: exclusive sums of the lengths of rows 0 .. rows (a last one of
@@ -172,26 +189,14 @@ __device__ __forceinline__ unsigned cta_exclusive(unsigned v, unsigned* total) {
   return before + inc - v;
 }
 
-constexpr int kCopies = 8;  // counters per row, or one
-__device__ __forceinline__ unsigned row_len(const unsigned* __restrict__ len, int copies,
-                                            long long n, long long k) {
-  unsigned v = __ldg(len + k);
-  if (copies == kCopies) {
-#pragma unroll
-    for (int c = 1; c < kCopies; ++c) v += __ldg(len + c * n + k);
-  }
-  return v;
-}
-
 __global__ void __launch_bounds__(kScanThreads)
-    block_sums_kernel(const unsigned* __restrict__ len, int copies, long long n,
-                      unsigned* __restrict__ sums) {
+    block_sums_kernel(const unsigned* __restrict__ len, long long n, unsigned* __restrict__ sums) {
   const long long base = (long long)blockIdx.x * kScan;
   unsigned v = 0;
 #pragma unroll
   for (int i = 0; i < kScanPer; ++i) {
     const long long k = base + i * kScanThreads + threadIdx.x;
-    v += k < n ? row_len(len, copies, n, k) : 0u;
+    v += k < n ? __ldg(len + k) : 0u;
   }
   unsigned total;
   cta_exclusive<kScanThreads>(v, &total);
@@ -210,7 +215,7 @@ __global__ void __launch_bounds__(1024) scan_sums_kernel(unsigned* sums, int n) 
 }
 
 __global__ void __launch_bounds__(kScanThreads)
-    apply_sums_kernel(const unsigned* __restrict__ len, int copies, long long n,
+    apply_sums_kernel(const unsigned* __restrict__ len, long long n,
                       const unsigned* __restrict__ sums, bool summed, uint2* __restrict__ row) {
   __shared__ unsigned s[kScan + kScan / 32];  // a word of padding per 32: conflict-free both ways
   auto at = [](int i) { return i + (i >> 5); };
@@ -220,7 +225,7 @@ __global__ void __launch_bounds__(kScanThreads)
 #pragma unroll
   for (int i = 0; i < kScanPer; ++i) {
     const long long k = base + i * kScanThreads + t;
-    mine[i] = k < n ? row_len(len, copies, n, k) : 0u;
+    mine[i] = k < n ? __ldg(len + k) : 0u;
     s[at(i * kScanThreads + t)] = mine[i];
   }
   __syncthreads();
@@ -560,10 +565,9 @@ el_status window_sort(el_workspace* w, const el_coo* coo, int32_t* offsets, int3
   const long long nnz = coo->nnz, rows = coo->rows, n = rows + 1;
   const int windows = (int)((nnz + Wn::W - 1) / Wn::W);
   const long long blocks = (n + kScan - 1) / kScan;
-  const int copies = nnz >= 4 * n ? kCopies : 1;
   // row length counters, window fills and flags (zeroed together), block
   // sums, rows (start, length), records
-  const size_t lbytes = round256((size_t)n * 4 * copies),
+  const size_t lbytes = round256((size_t)n * 4),
                fbytes = round256((size_t)(windows + 1) * kFillStride * 4),
                sbytes = round256((size_t)blocks * 4), rbytes = round256((size_t)n * 8);
   const size_t total = lbytes + fbytes + sbytes + rbytes + (size_t)windows * Wn::kCap * 16;
@@ -585,17 +589,18 @@ el_status window_sort(el_workspace* w, const el_coo* coo, int32_t* offsets, int3
   uint4* recs = reinterpret_cast<uint4*>(p + lbytes + fbytes + sbytes + rbytes);
   cudaError_t e = cudaMemsetAsync(p, 0, lbytes + fbytes, s);
   if (e != cudaSuccess) return cuda_status(e, "el_csr_from_coo");
-  const unsigned grid = (unsigned)std::min<long long>((nnz + 1023) / 1024, (long long)sms * 8);
+  const unsigned grid = (unsigned)std::min<long long>(
+      (nnz + 4 * kCountThreads - 1) / (4 * kCountThreads), (long long)sms * 2);
   if (rows <= kSmallRows)
-    count_rows_kernel<true><<<grid, 256, 0, s>>>(coo->row_indices, coo->col_indices, nnz, rows,
-                                                 coo->cols, len, copies, flags);
+    count_rows_kernel<true><<<grid, kCountThreads, 0, s>>>(
+        coo->row_indices, coo->col_indices, (int)nnz, (unsigned)rows, (unsigned)coo->cols, len, flags);
   else
-    count_rows_kernel<false><<<grid, 256, 0, s>>>(coo->row_indices, coo->col_indices, nnz, rows,
-                                                  coo->cols, len, copies, flags);
+    count_rows_kernel<false><<<grid, kCountThreads, 0, s>>>(
+        coo->row_indices, coo->col_indices, (int)nnz, (unsigned)rows, (unsigned)coo->cols, len, flags);
   const bool summed = blocks > kScanThreads;
-  if (blocks > 1) block_sums_kernel<<<(unsigned)blocks, kScanThreads, 0, s>>>(len, copies, n, sums);
+  if (blocks > 1) block_sums_kernel<<<(unsigned)blocks, kScanThreads, 0, s>>>(len, n, sums);
   if (summed) scan_sums_kernel<<<1, 1024, 0, s>>>(sums, (int)blocks);
-  apply_sums_kernel<<<(unsigned)blocks, kScanThreads, 0, s>>>(len, copies, n, sums, summed, row);
+  apply_sums_kernel<<<(unsigned)blocks, kScanThreads, 0, s>>>(len, n, sums, summed, row);
   const int msmem = kMoveTile * 16 + windows * 8;
   e = cudaFuncSetAttribute(move_kernel<LOGW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            kMoveTile * 16 + kMaxWindows * 8);

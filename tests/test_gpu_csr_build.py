@@ -2,7 +2,7 @@
 around a window (2048, 8192 places) and around the switch between the two,
 rows longer than a window's spare room, rows whose columns crowd together,
 many equal entries, windows that overfill (the radix sort takes over), mostly
-empty rows, entries already in order.  Equal to a stable sort by (row,
+empty rows, entries already in order, more rows than the count's tables hold.  Equal to a stable sort by (row,
 column), array for array."""
 import numpy as np
 import pytest
