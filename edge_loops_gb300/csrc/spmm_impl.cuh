@@ -39,6 +39,9 @@ constexpr int kFold = 32;           // steps (a power of two)
 // cost more to set apart than that saves.  Threshold none / 512 / 256 / 128:
 // 3,000 log-normal rows of 20, n = 9, 74 / 44 / 35 / 31 us; 60,000 of them,
 // n = 64, 93 / 70 / 64 / 64; 200,003 of 10, n = 24, 58 / 58 / 58 / 70.
+// Ranges of fewer items set shorter rows apart (launch_kernel): one row is
+// most of a warp's time there.  30,000 nonzeros in log-normal rows of 4, n = 4:
+// 32 us at 256, 17 at 64, 16 at 32; 300,000 in rows of 38: 20.0 / 20.0 / 17.9.
 constexpr int kLongRow = 256;
 // Merge items per row end: a row end costs the walk about two nonzeros (its
 // test, store and new sum).
@@ -62,6 +65,7 @@ struct Args {
   int n;  // columns in this pass
   long long range_items;  // merge items per warp
   int block_items;        // of them worked on at a time, at most kBlock
+  int long_row;           // ORDERED, several groups per warp: rows set apart from here on
   long long num_ranges;
   WsHeader* hdr;
   CarrySlot* flags;
@@ -176,7 +180,6 @@ struct Walk {
   using Sm = Smem<L, ORDERED>;
   static constexpr int G = L::G, U = L::U, NG = 32 / G, P = L::P, V = L::V, K = L::K;
   // (a block closes at most kBlock nonzeros beside its first row's)
-  static constexpr int kLong = NG > 1 ? kLongRow : kMaxNz - kBlock;
   const Args& a;
   Sm& M;
   const int lane, sl, grp;
@@ -335,7 +338,8 @@ struct Walk {
         if (i0 + 32 * u >= nrows) break;
         const int i = i0 + 32 * u + lane, s = s4[u], e = e4[u];
         if constexpr (ORDERED) {
-          const unsigned lm = __ballot_sync(kFullMask, i < nrows && e - s > kLong);
+          const int most = NG > 1 ? a.long_row : kMaxNz - kBlock;
+          const unsigned lm = __ballot_sync(kFullMask, i < nrows && e - s > most);
           if (lm) {  // the block ends before this row
             const int q = __ffs(lm) - 1;
             nrows = i0 + 32 * u + q;
@@ -771,6 +775,82 @@ __global__ void __launch_bounds__(kTPB, kMinCtas) spmm_kernel(const Args a) {
   }
 }
 
+// ------------------------------------------------------------- narrow B, C
+// thread_mapped with NC <= kNarrow columns: a thread per row, the row walked
+// once, W nonzeros' values and B elements in flight with the next W's
+// columns.  A B row is then less than the sectors it lies in, and rows of one
+// matrix row's neighbours share them in L1, while the row ends of the walk
+// above cost as much as for wide rows.  2M nonzeros, FP32, walk / thread per
+// row: 27-point stencil n = 1 29 / 15 us, n = 4 28 / 17; log-normal rows of 4
+// n = 4 59 / 49; uniform rows of 38 28 / 30.  From 6 columns on the walk is
+// faster on all of them.
+constexpr int kNarrow = 5;
+template <typename VT, typename BT, int NC>
+__global__ void __launch_bounds__(256, 3) thread_rows_kernel(const Args a) {
+  constexpr int W = NC == 1 ? 16 : 8;
+  const VT* const vals = reinterpret_cast<const VT*>(a.values);
+  for (long long row = (long long)blockIdx.x * blockDim.x + threadIdx.x; row < a.rows;
+       row += (long long)gridDim.x * blockDim.x) {
+    int b = __ldg(a.offsets + row), e = __ldg(a.offsets + row + 1);
+    if (b < 0 || e > a.nnz || e < b) {
+      raise_flag(a.hdr, EL_FLAG_OFFSETS, (unsigned)row);
+      b = min(max(b, 0), (int)a.nnz);
+      e = min(max(e, b), (int)a.nnz);
+    }
+    const float scale = a.row_scale ? __ldg(a.row_scale + row) : 1.f;
+    bool bad = false;
+    float sum[NC];
+    int c[W];
+#pragma unroll
+    for (int j = 0; j < NC; ++j) sum[j] = 0.f;
+    const int len = e - b;
+    const int* const idx = a.indices + b;
+    const VT* const val = vals + b;
+#pragma unroll
+    for (int k = 0; k < W; ++k) c[k] = k < len ? __ldg(idx + k) : -1;
+    for (int q = 0; q < len; q += W) {
+      float v[W], bv[W][NC];
+#pragma unroll
+      for (int k = 0; k < W; ++k) {
+        const bool ok = (unsigned)c[k] < (unsigned)a.cols;
+        bad |= !ok && k < len - q;
+        v[k] = ok ? to_f32(val[q + k]) : 0.f;
+        const BT* const r =
+            reinterpret_cast<const BT*>(a.B + (ok ? (unsigned)c[k] * a.ldb : 0ull));
+#pragma unroll
+        for (int j = 0; j < NC; ++j) bv[k][j] = ok ? to_f32(r[j]) : 0.f;
+      }
+#pragma unroll
+      for (int k = 0; k < W; ++k) c[k] = k < len - q - W ? __ldg(idx + q + W + k) : -1;
+#pragma unroll
+      for (int k = 0; k < W; ++k)
+        if (k < len - q) {
+#pragma unroll
+          for (int j = 0; j < NC; ++j) sum[j] = __fadd_rn(sum[j], __fmul_rn(v[k], bv[k][j]));
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < NC; ++j)
+      a.C[row * a.ldc + j] = a.row_scale ? sum[j] * scale : sum[j];
+    if (bad) raise_flag(a.hdr, EL_FLAG_INDEX_RANGE, (unsigned)row);
+  }
+}
+
+template <typename VT, typename BT>
+el_status launch_thread_rows(const SpmmCall& c, const Args& a) {
+  const long long most = (long long)device_info(c.device).sm_count * 32;
+  const long long need = (a.rows + 255) / 256;
+  const unsigned grid = (unsigned)(need < most ? need : most);
+  switch (a.n) {
+    case 1: thread_rows_kernel<VT, BT, 1><<<grid, 256, 0, c.stream>>>(a); break;
+    case 2: thread_rows_kernel<VT, BT, 2><<<grid, 256, 0, c.stream>>>(a); break;
+    case 3: thread_rows_kernel<VT, BT, 3><<<grid, 256, 0, c.stream>>>(a); break;
+    case 4: thread_rows_kernel<VT, BT, 4><<<grid, 256, 0, c.stream>>>(a); break;
+    default: thread_rows_kernel<VT, BT, kNarrow><<<grid, 256, 0, c.stream>>>(a); break;
+  }
+  return cuda_status(cudaGetLastError(), "spmm launch");
+}
+
 // ----------------------------------------------------------------- launch
 template <typename L, bool ORDERED>
 el_status launch_kernel(const SpmmCall& c, Args a) {
@@ -789,6 +869,7 @@ el_status launch_kernel(const SpmmCall& c, Args a) {
   a.range_items = ri;
   const long long blocks = (ri + kBlock - 1) / kBlock;
   a.block_items = (int)((ri + blocks - 1) / blocks);
+  a.long_row = ri >= kLongRow ? kLongRow : ri > 128 ? (int)ri / 4 : 32;
   a.num_ranges = (total + ri - 1) / ri;
   const long long grid = (a.num_ranges + kWarps - 1) / kWarps;
   kern<<<(unsigned)grid, kTPB, 0, c.stream>>>(a);
@@ -821,6 +902,18 @@ el_status launch(const SpmmCall& c, int schedule) {
   a.flags = c.ws.slots;
   a.vec = reinterpret_cast<float*>(c.scratch);
   a.wait_ns = c.wait_ns;
+  if (schedule == EL_SCHED_THREAD_MAPPED && c.n <= kNarrow) {
+    a.n = (int)c.n;
+    a.b_first = 0;
+    a.C = c.C;
+    if (a.value_dtype == EL_F32) return launch_thread_rows<float, BT>(c, a);
+    if constexpr (kB == 4) {
+      return a.value_dtype == EL_BF16 ? launch_thread_rows<__nv_bfloat16, BT>(c, a)
+                                      : launch_thread_rows<__half, BT>(c, a);
+    } else {  // 16-bit values come with B of their own type alone
+      return launch_thread_rows<BT, BT>(c, a);
+    }
+  }
   // columns per load: the widest vectors on whose boundaries every row of B
   // and C starts and of which n is a multiple
   int v = 16 / kB;

@@ -178,3 +178,28 @@ def test_keeps_a_captured_spmv(cuda, ragged):
     g.replay()
     torch.cuda.synchronize()
     assert ws.errors() == 0 and torch.equal(y.cpu(), exp) and bool(C.isfinite().all())
+
+
+@pytest.mark.parametrize("vdt,bdt", [("f32", "f32"), ("bf16", "f32"), ("f16", "f32"),
+                                     ("bf16", "bf16"), ("f16", "f16"), ("f32", "f16")])
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 6])
+def test_narrow_thread_mapped(cuda, oracle_mod, ragged, n, vdt, bdt):
+    """A thread per row up to 5 columns: rows of 0 .. 12,000 nonzeros, all value
+    and B types, scales; equal to the reference loop bit for bit."""
+    from edge_loops_gb300 import api
+    off, idx, vals = ragged
+    dt = {"f32": torch.float32, "bf16": torch.bfloat16, "f16": torch.float16}
+    g = torch.Generator(device=cuda)
+    g.manual_seed(n)
+    B = (torch.rand(20_000, n, device=cuda, generator=g) * 2 - 1).to(dt[bdt])
+    A = api.CSR.from_arrays(off, idx, vals, 20_000, device=cuda)
+    scale = None
+    if vdt != "f32":
+        A = A.quantized(dt[vdt])
+        scale = A.row_scale.cpu().numpy()
+    C = api.spmm(A, B, schedule="thread_mapped")
+    assert api.workspace_errors() == 0
+    exp = oracle_mod.spmm_f32(off, idx, A.values.float().cpu().numpy(), as_f32(B))
+    if scale is not None:
+        exp = exp * scale[:, None]  # powers of two: exact
+    np.testing.assert_array_equal(C.cpu().numpy(), exp)
