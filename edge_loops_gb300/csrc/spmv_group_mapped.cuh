@@ -51,13 +51,14 @@ el_status launch_group_mapped_rows(const SpmvCall& c, int group_rows) {
   Src m{c.A.offsets, c.A.indices, c.A.values, c.A.row_scale, c.x, c.y,
         (int)c.A.rows, (unsigned)c.A.cols, (int)c.A.nnz, 0, 0};
   tile_phase(c.A.indices, c.A.values, (int)sizeof(VT), &m.vec_ok, &m.ph);
-  // A warp takes the whole group where that leaves 1.5 chunks per resident
-  // warp, else fewer rows, down to 32: whole tiles against warps left idle.
+  // A warp takes the whole group (four together where a group is 32 rows)
+  // where that leaves 1.5 chunks per resident warp, else fewer rows, down to
+  // 32: whole tiles against warps left idle.
   // 32 / 64 / 128 rows per warp: stencil 96^3 (885k rows) 76 / 64 / 60 us,
   // 2M log-normal rows of 8 117 / 101 / 91, stencil 40^3 (64k rows) 15 / 17 /
   // 25, 100k uniform rows of 35 25 / 29 / 31 (a block scan per 128 nonzeros:
   // 191, 156, 29, 48).
-  int rpw = group_rows;
+  int rpw = group_rows > 128 ? group_rows : 128;
   while (rpw > 32 && c.A.rows * 2 < 3 * ctas * kWarps * rpw) rpw /= 2;
   const long long chunks = (c.A.rows + rpw - 1) / rpw;
   long long grid = (chunks + kWarps - 1) / kWarps;
