@@ -778,12 +778,12 @@ __global__ void __launch_bounds__(kTPB, kMinCtas) spmm_kernel(const Args a) {
 // ------------------------------------------------------------- narrow B, C
 // thread_mapped with NC <= kNarrow columns: a thread per row, the row walked
 // once, W nonzeros' values and B elements in flight with the next W's
-// columns.  A B row is then less than the sectors it lies in, and rows of one
-// matrix row's neighbours share them in L1, while the row ends of the walk
-// above cost as much as for wide rows.  2M nonzeros, FP32, walk / thread per
-// row: 27-point stencil n = 1 29 / 15 us, n = 4 28 / 17; log-normal rows of 4
-// n = 4 59 / 49; uniform rows of 38 28 / 30.  From 6 columns on the walk is
-// faster on all of them.
+// columns.  A B row is then less than the sectors it lies in, neighbouring
+// rows of a banded matrix share them in L1, and the row ends of the walk above
+// cost as much as for wide rows.  2M nonzeros, FP32, walk / thread per row:
+// 27-point stencil n = 1 29 / 10 us, n = 4 28 / 14; n = 4 in log-normal rows of
+// 4 59 / 32, uniform rows of 38 28 / 30, log-normal rows of 38 77 / 98.  From 6
+// columns on the walk is faster.
 constexpr int kNarrow = 5;
 template <typename VT, typename BT, int NC>
 __global__ void __launch_bounds__(256, 3) thread_rows_kernel(const Args a) {

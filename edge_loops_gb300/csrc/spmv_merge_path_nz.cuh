@@ -509,25 +509,16 @@ using NzWalk = NzWalkK<kPer>;
 // The sum of the partials that ranges [gfirst, g) published of the row they
 // leave open, in a fixed order (a warp's work; bounded waits: ok = false when
 // one ran out).
-template <bool COMP, int kBatch = 8>
+template <bool COMP>
 __device__ __forceinline__ Acc<COMP> look_back(const Args& a, long long gfirst, long long g,
                                                unsigned tag, bool& ok) {
   const int lane = threadIdx.x & 31;
   Acc<COMP> acc;
   ok = true;
   if (gfirst < 0) gfirst = 0;  // malformed offsets
-  const long long gend = g < a.ws.nslots ? g : a.ws.nslots;
-  // kBatch flags at a time, then their partials: a row of 2M nonzeros lies in
-  // 3648 ranges (one at a time: 57 us, of which the look-back took most).
-  for (long long kk = gfirst + lane; kk < gend && ok; kk += 32 * kBatch) {
-    unsigned missing = 0;
-#pragma unroll
-    for (int i = 0; i < kBatch; ++i)
-      if (kk + 32 * i < gend &&
-          *reinterpret_cast<volatile unsigned*>(&a.ws.slots[kk + 32 * i].flag) != tag)
-        missing |= 1u << i;
-    for (; missing && ok; missing &= missing - 1) {
-      const CarrySlot* sl = a.ws.slots + kk + 32 * (__ffs(missing) - 1);
+  for (long long kk = gfirst + lane; kk < g && kk < a.ws.nslots; kk += 32) {
+    CarrySlot* sl = a.ws.slots + kk;
+    if (ld_acquire_u32(&sl->flag) != tag) {
       const uint64_t t0 = global_timer_ns();
       while (ld_acquire_u32(&sl->flag) != tag) {
         if (global_timer_ns() - t0 > a.wait_ns) {
@@ -538,15 +529,9 @@ __device__ __forceinline__ Acc<COMP> look_back(const Args& a, long long gfirst, 
       }
     }
     if (!ok) break;
-    __threadfence();  // the flags before the partials
-    Acc<COMP> pv[kBatch];
-#pragma unroll
-    for (int i = 0; i < kBatch; ++i)
-      if (kk + 32 * i < gend)
-        pv[i].set(__ldcg(&a.ws.slots[kk + 32 * i].sum), __ldcg(&a.ws.slots[kk + 32 * i].comp));
-#pragma unroll
-    for (int i = 0; i < kBatch; ++i)
-      if (kk + 32 * i < gend) acc.add(pv[i]);
+    Acc<COMP> pv;
+    pv.set(__ldcg(&sl->sum), __ldcg(&sl->comp));
+    acc.add(pv);
   }
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) {

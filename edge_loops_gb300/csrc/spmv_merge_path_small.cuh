@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(kSmTPB) merge_path_small_kernel(const Args a) 
     float s = warp_sum(min(max(S.off[ob + i] - n0, 0), e), e);
     if (i == 0 && inside && !again) {
       bool ok;
-      Acc<false> acc = look_back<false, 1>(a, (w * rs + sa.start) / a.range_items, g, tag, ok);
+      Acc<false> acc = look_back<false>(a, (w * rs + sa.start) / a.range_items, g, tag, ok);
       if (!ok && lane == 0) raise_flag(hdr, EL_FLAG_TIMEOUT, 4);
       s = __fadd_rn(acc.s, s);
     }

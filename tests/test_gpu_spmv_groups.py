@@ -96,6 +96,29 @@ def test_many_threads_under_capture(cuda, oracle_mod, num_threads):
     assert np.all(np.abs(y.cpu().numpy() - y64) <= order_free_bound(off, yabs))
 
 
+@pytest.mark.parametrize("sched,opts", [
+    ("merge_path_flat", {"nz_per_lane": 8}), ("merge_path_flat", {"compensated": True}),
+    ("work_oriented", {}), ("work_oriented", {"num_threads": 9600}), ("group_mapped", {})],
+    ids=lambda v: str(v))
+@pytest.mark.parametrize("n", [70_000, 1_300_000])
+def test_row_of_many_ranges(cuda, oracle_mod, n, sched, opts):
+    """One row in up to some thousand ranges, between short ones."""
+    from edge_loops_gb300 import api
+    rng = np.random.default_rng(n)
+    lens = np.concatenate([np.full(50, 3), [n], np.full(50, 2)])
+    off = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    idx = rng.integers(0, 5000, size=off[-1]).astype(np.int32)
+    vals = rng.uniform(-1, 1, size=off[-1]).astype(np.float32)
+    x = rng.uniform(-1, 1, size=5000).astype(np.float32)
+    A = api.CSR.from_arrays(off, idx, vals, 5000, device=cuda)
+    y64, yabs = oracle_mod.spmv_f64(off, idx, vals, x)
+    got = [api.spmv(A, torch.as_tensor(x, device=cuda), schedule=sched, **opts).cpu().numpy()
+           for _ in range(2)]
+    assert api.workspace_errors() == 0
+    np.testing.assert_array_equal(got[0], got[1])
+    assert np.all(np.abs(got[0] - y64) <= order_free_bound(off, yabs))
+
+
 def test_num_threads_is_checked(cuda):
     from edge_loops_gb300 import _lib, api
     off, idx, vals, x = case("rows33")
