@@ -331,6 +331,14 @@ struct SplitPoint {
   int start;    // offsets[x]
   int end;      // offsets[x + 1] (nnz for x == rows)
 };
+// The split point's nonzero coordinate on diagonal d, inside [0, nnz] whatever
+// the offsets hold (on well-formed ones the bounds change nothing).
+__device__ __forceinline__ int split_nonzero(const SplitPoint& S, long long d, long long w,
+                                             long long rows, long long nnz) {
+  long long n = d - w * S.x;
+  if (S.x < rows) n = min(n, (long long)S.end);
+  return (int)min(max(n, 0LL), nnz);
+}
 // `row_end(k)` reads offsets[k + 1], k >= -1.
 template <typename RowEnd>
 __device__ __forceinline__ void warp_merge_search2_w(const RowEnd& row_end, long long rows,

@@ -580,14 +580,10 @@ __device__ __forceinline__ void run_range(const Args& a, SmemT& S, const int war
     SplitPoint sa, sb;
     warp_merge_search2_w([&](long long k) { return __ldg(a.offsets + 1 + k); }, a.rows, a.nnz, d0,
                          d1, w, sa, sb);
-    auto nz_of = [&](long long d, const SplitPoint& sp) {  // the nonzero coordinate
-      const long long n = d - w * sp.x;
-      return (int)(sp.x < a.rows ? min(n, (long long)sp.end) : n);
-    };
     const int rs = (int)sa.x;
-    const int ns = nz_of(d0, sa);
+    const int ns = split_nonzero(sa, d0, w, a.rows, a.nnz);
     const int re = (int)sb.x;
-    const int ne = nz_of(d1, sb);
+    const int ne = split_nonzero(sb, d1, w, a.rows, a.nnz);
     const int off_rs = sa.start;
     const bool need_lb = ns > off_rs;
     if (a.trace && g < a.trace_cap && lane < 6) {

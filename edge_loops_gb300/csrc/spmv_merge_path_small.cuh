@@ -68,11 +68,9 @@ __global__ void __launch_bounds__(kSmTPB) merge_path_small_kernel(const Args a) 
     sa = S.sp[0];
     sb = S.sp[1];
   }
-  auto nz_of = [&](long long d, const SplitPoint& sp) {  // the nonzero coordinate
-    const long long n = d - w * sp.x;
-    return (int)(sp.x < a.rows ? min(n, (long long)sp.end) : n);
-  };
-  const int rs = (int)sa.x, re = (int)sb.x, ns = nz_of(d0, sa), ne = nz_of(d1, sb);
+  const int rs = (int)sa.x, re = (int)sb.x;
+  const int ns = split_nonzero(sa, d0, w, a.rows, a.nnz);
+  const int ne = split_nonzero(sb, d1, w, a.rows, a.nnz);
   if (a.trace && g < a.trace_cap && t < 6) {
     const long long t6[6] = {d0, d1, rs, ns, re, ne};
     long long tv = t6[0];
