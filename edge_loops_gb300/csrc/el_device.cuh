@@ -329,15 +329,16 @@ __device__ __forceinline__ long long warp_merge_search(
 struct SplitPoint {
   long long x;  // rows closed before the diagonal
   int start;    // offsets[x]
-  int end;      // offsets[x + 1] (nnz for x == rows)
+  int end;      // offsets[x + 1] (nnz for x == rows), inside [0, nnz] whatever it holds
 };
-// The split point's nonzero coordinate on diagonal d, inside [0, nnz] whatever
-// the offsets hold (on well-formed ones the bounds change nothing).
+// The split point's nonzero coordinate on diagonal d <= w rows + nnz.  Inside
+// [0, nnz] whatever the offsets hold: 0 <= d - w x (x <= d / w), at most nnz
+// where x == rows, and S.end is bounded.  (Bounding the coordinate instead of
+// the end costs the SpMM walk, n = 128, 410 us for 400: other registers.)
 __device__ __forceinline__ int split_nonzero(const SplitPoint& S, long long d, long long w,
-                                             long long rows, long long nnz) {
-  long long n = d - w * S.x;
-  if (S.x < rows) n = min(n, (long long)S.end);
-  return (int)min(max(n, 0LL), nnz);
+                                             long long rows) {
+  const long long n = d - w * S.x;
+  return (int)(S.x < rows ? min(n, (long long)S.end) : n);
 }
 // `row_end(k)` reads offsets[k + 1], k >= -1.
 template <typename RowEnd>
@@ -391,6 +392,7 @@ __device__ __forceinline__ void warp_merge_search2_w(const RowEnd& row_end, long
     const int ve = __shfl_sync(kFullMask, v[k], c < 32 ? c : 31);
     const int vs = __shfl_sync(kFullMask, v[k], c > 0 ? c - 1 : 0);
     S.end = (S.x < hi[k] && c < 32) ? ve : S.x < rows ? row_end(S.x) : (int)nnz;
+    S.end = min(max(S.end, 0), (int)nnz);
     S.start = c > 0 ? vs : S.x > 0 ? row_end(S.x - 1) : row_end(-1);
   }
 }

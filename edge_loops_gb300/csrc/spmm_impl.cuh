@@ -46,6 +46,7 @@ constexpr int kLongRow = 256;
 // Merge items per row end: a row end costs the walk about two nonzeros (its
 // test, store and new sum).
 constexpr int kRowItems = 2;
+constexpr int kMaxRows = kBlock / kRowItems + 1;  // rows of a block, at most
 // Resident CTAs per SM: 24 warps of 80 registers (8M nonzeros, n = 32: 187 µs;
 // 20 warps of 96: 205; 32 of 64, which spills in the walk: 230).
 constexpr int kMinCtas = 6;
@@ -161,7 +162,7 @@ struct Smem {  // per warp
   __align__(16) float val[2][32];  // and values
   float sc[2][32];                 // scales of the G rows from the step's first on
   unsigned ends[kMaxNz / 32 + 4];  // bit i: a row ends after the block's nonzero i
-  unsigned rowm[kBlock / 32 + 4];  // bit i: row i of the block ends by such a bit
+  unsigned rowm[kMaxRows / 32 + 4];  // bit i: row i of the block ends by such a bit
   float open[ORDERED ? 1 : NG][ORDERED ? 1 : L::kCols];  // a piece's open row
   float pend[ORDERED ? 1 : NG][ORDERED ? 1 : L::kCols];  // its part of the row it began inside
   float fold[ORDERED ? 1 : L::P][32];  // the lanes' earlier sums of a long row
@@ -300,10 +301,12 @@ struct Walk {
     __syncwarp();
   }
 
-  // One block: rows [rs, re) and nonzeros [ns, ne), the rows' ends among
-  // them.  `inside`: row rs began before nonzero ns.  z_out: row rs ends here
-  // without a nonzero.  ORDERED: stops before the first long row; returns the
-  // row it stopped at.
+  // One block: rows [rs, re), at most kMaxRows, and nonzeros [ns, ne), the rows'
+  // ends among them (not ORDERED: at most kMaxNz).  `inside`: row rs began before
+  // nonzero ns.  z_out: row rs ends here without a nonzero.  ORDERED: stops
+  // before the first row that is long or whose offsets fall or leave [ns, ne], so
+  // that the rows before it have distinct ends in order; returns the row it
+  // stopped at.
   // Leaves every piece's open row in M.open, with M.first, closed, has_pend.
   __device__ __forceinline__ int block(const int rs, int re, const int ns, int ne,
                                        const bool inside, bool& z_out) {
@@ -339,7 +342,10 @@ struct Walk {
         const int i = i0 + 32 * u + lane, s = s4[u], e = e4[u];
         if constexpr (ORDERED) {
           const int most = NG > 1 ? a.long_row : kMaxNz - kBlock;
-          const unsigned lm = __ballot_sync(kFullMask, i < nrows && e - s > most);
+          const bool off = i < nrows && (s < ns || e < s || e > ne);
+          bad_off |= off;
+          const unsigned lm = __ballot_sync(
+              kFullMask, i < nrows && (off || e - s > most || e - ns > kMaxNz));
           if (lm) {  // the block ends before this row
             const int q = __ffs(lm) - 1;
             nrows = i0 + 32 * u + q;
@@ -353,7 +359,7 @@ struct Walk {
           const unsigned m = 1u << ((e - ns - 1) & 31);
           bad_off |= (atomicOr(&M.ends[(e - ns - 1) >> 5], m) & m) != 0;
         }
-        bad_off |= i < nrows && !empty && !z && (!bit || e < s || (ORDERED && s < ns));
+        bad_off |= i < nrows && !empty && !z && (!bit || e < s);
         z_out |= __any_sync(kFullMask, z);
         const unsigned rb = __ballot_sync(kFullMask, bit);
         if (lane == 0) M.rowm[i >> 5] = rb;
@@ -368,9 +374,9 @@ struct Walk {
     __syncwarp();
     if (ORDERED) {
       re = rs + nrows;
+      if (nrows == 0) return re;
+      ne = min(ne, ns + kMaxNz);  // (past the last row's end on malformed offsets alone)
       len = ne - ns;
-      if (len > kMaxNz) bad_off = true;  // malformed offsets
-      if (nrows == 0 || len > kMaxNz) return re;
       per = share();
     }
 
@@ -650,14 +656,14 @@ __global__ void __launch_bounds__(kTPB, kMinCtas) spmm_kernel(const Args a) {
     const long long db = min(d + a.block_items, d1);
     warp_merge_search2_w([&](long long k) { return __ldg(a.offsets + 1 + k); }, a.rows, a.nnz, d,
                          db, kRowItems, sa, sb);
-    auto nz_of = [&](long long dd, const SplitPoint& sp) {  // the nonzero coordinate
-      const long long n = dd - kRowItems * sp.x;
-      return (int)(sp.x < a.rows ? min(n, (long long)sp.end) : n);
-    };
-    int rs = (int)sa.x, ns = nz_of(d, sa);
+    int rs = (int)sa.x, ns = split_nonzero(sa, d, kRowItems, a.rows);
     re = (int)sb.x;
-    ne = nz_of(db, sb);
+    ne = split_nonzero(sb, db, kRowItems, a.rows);
     off_re = sb.start;
+    // on malformed offsets the two split points are unrelated
+    const int re_in = min(max(re, rs), rs + kMaxRows);
+    if (re != re_in) raise_flag(a.hdr, EL_FLAG_OFFSETS, (unsigned)rs);
+    re = re_in;
     bool z = false;
     if (ORDERED) {  // whole rows
       const int m = (int)a.nnz;
@@ -676,6 +682,9 @@ __global__ void __launch_bounds__(kTPB, kMinCtas) spmm_kernel(const Args a) {
         n0 = ns;
         off_r0 = sa.start;
       }
+      const int ne_in = min(max(ne, ns), ns + kMaxNz);
+      if (ne != ne_in) raise_flag(a.hdr, EL_FLAG_OFFSETS, (unsigned)rs);
+      ne = ne_in;
       walk.block(rs, re, ns, ne, ns > sa.start, z);
       // stitch the rows that cross pieces, in piece order
       const bool need_lb = n0 > off_r0;

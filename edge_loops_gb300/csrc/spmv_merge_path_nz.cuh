@@ -581,9 +581,9 @@ __device__ __forceinline__ void run_range(const Args& a, SmemT& S, const int war
     warp_merge_search2_w([&](long long k) { return __ldg(a.offsets + 1 + k); }, a.rows, a.nnz, d0,
                          d1, w, sa, sb);
     const int rs = (int)sa.x;
-    const int ns = split_nonzero(sa, d0, w, a.rows, a.nnz);
+    const int ns = split_nonzero(sa, d0, w, a.rows);
     const int re = (int)sb.x;
-    const int ne = split_nonzero(sb, d1, w, a.rows, a.nnz);
+    const int ne = split_nonzero(sb, d1, w, a.rows);
     const int off_rs = sa.start;
     const bool need_lb = ns > off_rs;
     if (a.trace && g < a.trace_cap && lane < 6) {

@@ -69,8 +69,8 @@ __global__ void __launch_bounds__(kSmTPB) merge_path_small_kernel(const Args a) 
     sb = S.sp[1];
   }
   const int rs = (int)sa.x, re = (int)sb.x;
-  const int ns = split_nonzero(sa, d0, w, a.rows, a.nnz);
-  const int ne = split_nonzero(sb, d1, w, a.rows, a.nnz);
+  const int ns = split_nonzero(sa, d0, w, a.rows);
+  const int ne = split_nonzero(sb, d1, w, a.rows);
   if (a.trace && g < a.trace_cap && t < 6) {
     const long long t6[6] = {d0, d1, rs, ns, re, ne};
     long long tv = t6[0];

@@ -68,3 +68,40 @@ def test_spmv_stays_inside(cuda, oracle_mod, rows, schedule, opts):
         y64, yabs = oracle_mod.spmv_f64(A.offsets.cpu().numpy(), A.indices.cpu().numpy(),
                                         A.values.cpu().numpy(), x.cpu().numpy())
         assert np.all(np.abs(y.cpu().numpy() - y64) <= 12 * 2.0 ** -24 * yabs)
+
+
+@pytest.mark.parametrize("schedule", ["merge_path", "thread_mapped", "group_mapped"])
+@pytest.mark.parametrize("n,bdt", [(4, "f32"), (8, "f32"), (24, "f32"), (32, "bf16"), (128, "f32")])
+@pytest.mark.parametrize("rows", [300, 6000, 60_000])
+def test_spmm_stays_inside(cuda, oracle_mod, rows, n, bdt, schedule):
+    """60,000 rows: the two split points of a block lie up to thousands of rows
+    apart where the offsets are not monotone."""
+    from edge_loops_gb300 import api
+    rng = np.random.default_rng(rows + n)
+    ws = api.Workspace()
+    B = torch.as_tensor(rng.uniform(-1, 1, (COLS, n)).astype(np.float32), device=cuda)
+    B = B.to(torch.bfloat16) if bdt == "bf16" else B
+    for kind in KINDS:
+        A, C = check(lambda A, C: api.spmm(A, B, C.view(rows, n), schedule=schedule, workspace=ws,
+                                           wait_limit_us=2000),
+                     ws, n, kind, rows, rng, cuda)
+    off, idx, vals = (t.cpu().numpy() for t in (A.offsets, A.indices, A.values))
+    got, Bf = C.view(rows, n).cpu().numpy(), B.float().cpu().numpy()
+    if schedule == "merge_path":
+        C64, Ca = oracle_mod.spmm_f64(off, idx, vals, Bf)
+        assert np.all(np.abs(got - C64) <= 12 * 2.0 ** -24 * Ca)
+    else:
+        np.testing.assert_array_equal(got, oracle_mod.spmm_f32(off, idx, vals, Bf))
+
+
+@pytest.mark.parametrize("schedule", ["merge_path", "thread_mapped", "group_mapped"])
+@pytest.mark.parametrize("kind", ["negative", "too large", "random"])
+def test_spmm_flags_bad_offsets(cuda, kind, schedule):
+    from edge_loops_gb300 import _lib, api
+    rng = np.random.default_rng(11)
+    ws = api.Workspace()
+    A = matrix(kind, 6000, rng, cuda)
+    api.spmm(A, torch.rand(COLS, 24, device=cuda), schedule=schedule, workspace=ws,
+             wait_limit_us=2000)
+    torch.cuda.synchronize()
+    assert ws.errors() & _lib.EL_FLAG_OFFSETS

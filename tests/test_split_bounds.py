@@ -34,10 +34,9 @@ def split(off, rows, nnz, d, w):
 
 
 def nonzero(x, end, d, w, rows, nnz):
-    """split_nonzero, and the coordinate before its bounds."""
+    """split_nonzero of the bounded end, and of the end as the offsets have it."""
     n = d - w * x
-    raw = min(n, end) if x < rows else n
-    return min(max(raw, 0), nnz), raw
+    return tuple(min(n, e) if x < rows else n for e in (min(max(end, 0), nnz), end))
 
 
 def ranges(off, nnz, w, items):
@@ -91,7 +90,7 @@ KINDS = ["negative", "first row", "int min", "too large", "int max", "falls", "r
 
 def test_every_range_stays_inside():
     rng = np.random.default_rng(3)
-    outside = set()  # kinds whose coordinates leave [0, nnz] before the bounds
+    outside = set()  # kinds whose coordinates leave [0, nnz] without the bounds
     for kind in KINDS:
         for rows in (7, 300, 6000):
             for trial in range(12 if rows < 6000 else 3):
@@ -128,3 +127,120 @@ def test_kernels_take_the_bounded_coordinate(source):
         text = f.read()
     assert text.count("split_nonzero(") == 2
     assert "sp.end" not in text and "sa.end" not in text and "sb.end" not in text
+
+
+# ------------------------------------------------------------------- SpMM
+BLOCK, MAX_NZ, ROW_ITEMS = 4096, 8192, 2  # spmm_impl.cuh
+MAX_ROWS = BLOCK // ROW_ITEMS + 1
+ENDS_WORDS, ROWM_WORDS = MAX_NZ // 32 + 4, MAX_ROWS // 32 + 4
+
+
+def spmm_block(off, nnz, rs, re, ns, ne, inside, ordered, groups, u, long_row):
+    """Walk::block: asserts what it reads and writes; the row it stops at."""
+    rows = len(off) - 1
+    assert 0 <= rs <= re <= rows and re - rs <= MAX_ROWS and 0 <= ns <= ne <= nnz
+    assert ordered or ne - ns <= MAX_NZ
+    nrows, length = re - rs, ne - ns
+    assert (min(length, MAX_NZ) >> 5) + 2 <= ENDS_WORDS and (nrows >> 5) + 2 <= ROWM_WORDS
+    if ordered:
+        for i in range(nrows):
+            s, e = int(off[rs + i]), int(off[rs + i + 1])
+            if s < ns or e < s or e > ne or e - s > long_row or e - ns > MAX_NZ:
+                nrows, ne = i, min(max(s, ns), ne)
+                break
+    ends, rowm, z_out = set(), [], False
+    for i in range(nrows):
+        s, e = int(off[rs + i]), int(off[rs + i + 1])
+        z = not ordered and i == 0 and inside and e == ns
+        z_out |= z
+        if s != e and not z and ns < e <= ne and e - ns <= MAX_NZ:
+            assert 0 <= (e - ns - 1) >> 5 < ENDS_WORDS
+            ends.add(e - ns - 1)
+            rowm.append(i)
+    if ordered:
+        re = rs + nrows
+        if nrows == 0:
+            return re
+        ne = min(ne, ns + MAX_NZ)
+    length = ne - ns
+    per = -(-length // (groups * u)) * u
+    dense = len(rowm) == nrows
+    pieces = []
+    for g in range(groups):
+        q = min(per * g, length)
+        assert (q >> 5) < ENDS_WORDS
+        before = sum(e < q for e in ends)
+        k = before if dense else (rowm[before] if before < len(rowm) else nrows)
+        pieces.append((min(k, nrows) if not dense else k, ns + q))
+    for g, (k, y) in enumerate(pieces):
+        if ordered:  # whole rows, from row k's start to the next piece's row's
+            def start(j):
+                return min(max(int(off[rs + j]), ns), ne) if j < nrows else ne
+            y = start(k)
+            ye = max(start(pieces[g + 1][0]) if g + 1 < groups else ne, y)
+        else:
+            ye = min(y + per, ne)
+        assert 0 <= y <= ye <= nnz and ye - ns <= MAX_NZ  # indices, values, M.ends
+        for e in sorted(e for e in ends if y - ns <= e < ye - ns):
+            assert k < nrows, "a store past the block's rows"
+            k = k + 1 if dense else next((r for r in rowm if r > k), nrows)
+    return re
+
+
+def spmm_range(off, nnz, items, ordered, groups, u, long_row):
+    """Every warp range of spmm_kernel, in blocks."""
+    rows = len(off) - 1
+    total = ROW_ITEMS * rows + nnz
+    n_blocks = -(-items // BLOCK)
+    block_items = -(-items // n_blocks)
+    for d0 in range(0, total, items):
+        d1 = min(d0 + items, total)
+        for d in range(d0, d1, block_items):
+            db = min(d + block_items, d1)
+            rs, start, end = split(off, rows, nnz, d, ROW_ITEMS)
+            re, start1, end1 = split(off, rows, nnz, db, ROW_ITEMS)
+            ns = nonzero(rs, end, d, ROW_ITEMS, rows, nnz)[0]
+            ne = nonzero(re, end1, db, ROW_ITEMS, rows, nnz)[0]
+            re = min(max(re, rs), rs + MAX_ROWS)
+            if not ordered:
+                ne = min(max(ne, ns), ns + MAX_NZ)
+                spmm_block(off, nnz, rs, re, ns, ne, ns > start, False, groups, u, long_row)
+                continue
+            ns = min(max(start, 0), nnz)
+            ne = min(max(start1, ns), nnz)
+            while rs < re:
+                rs = spmm_block(off, nnz, rs, re, ns, ne, False, True, groups, u, long_row)
+                if rs >= re:
+                    break
+                b = min(max(int(off[rs]), ns), ne)
+                ns = min(max(int(off[rs + 1]), b), ne)
+                assert 0 <= b <= ns <= nnz  # the long row's nonzeros
+                rs += 1
+
+
+@pytest.mark.parametrize("ordered", [False, True])
+@pytest.mark.parametrize("groups,u", [(8, 4), (4, 8), (1, 8)])
+def test_spmm_blocks_stay_inside(ordered, groups, u):
+    rng = np.random.default_rng(5)
+    for kind in KINDS + ["none"]:
+        for rows, items in ((300, 64), (6000, 512), (6000, 9000), (9000, 4096)):
+            off, nnz = offsets(kind, rng, rows)
+            spmm_range(off, nnz, items, ordered, groups, u, 256 if groups > 1 else BLOCK)
+
+
+def test_spmm_rows_of_two_split_points_were_unbounded():
+    """What the bound on a block's rows is for: split points of offsets that
+    are not monotone lie far apart."""
+    off, nnz = offsets("random", np.random.default_rng(6), 60_000)
+    most = 0
+    for d in range(0, 2 * 60_000 + nnz - 4096, 4096):
+        rs = split(off, 60_000, nnz, d, 2)[0]
+        most = max(most, split(off, 60_000, nnz, d + 4096, 2)[0] - rs)
+    assert most > 32 * ROWM_WORDS
+
+
+def test_spmm_takes_the_bounded_coordinate():
+    with open(os.path.join(CSRC, "spmm_impl.cuh")) as f:
+        text = f.read()
+    assert text.count("split_nonzero(") == 2 and "sp.end" not in text
+    assert "min(max(re, rs), rs + kMaxRows)" in text and "min(max(ne, ns), ns + kMaxNz)" in text
