@@ -763,6 +763,9 @@ __global__ void __launch_bounds__(kTPB, kMinCtas) spmm_kernel(const Args a) {
         }
         ok = __all_sync(kFullMask, ok);
         if (!ok) break;
+        // the lanes' acquires come before every lane's reads of the vectors
+        // (a vote alone orders no memory)
+        __syncwarp();
         const int cnt = (int)(w - base < 32 ? w - base : 32);
 #pragma unroll 8
         for (int k = 0; k < cnt; ++k) {
