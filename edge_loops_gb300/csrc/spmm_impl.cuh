@@ -462,8 +462,10 @@ struct Walk {
 #pragma unroll
     for (int k = 0; k < P; ++k) acc[k] = 0.f;
     bool has_pend = false;
-    // a long row's sum is put aside every kFold steps without a row end: short
-    // chains of additions, for the rounding error
+    // a row's sum is put aside in every kFold-th step unless the row's group has a
+    // row end in it: short chains of additions, for the rounding error (a row
+    // that begins in such a step waits for the next: at most (kFold + 1) U - 1
+    // nonzeros in one chain)
     bool folded = false;
     auto unfold = [&]() {
       if constexpr (!ORDERED) {
@@ -531,16 +533,6 @@ struct Walk {
       if (!__any_sync(kFullMask, ends != 0)) {
 #pragma unroll
         for (int j = 0; j < U; ++j) add(v[j], b[j], acc);
-        if constexpr (!ORDERED) {
-          if ((i & (kFold - 1)) == kFold - 1) {
-#pragma unroll
-            for (int k = 0; k < P; ++k) {
-              M.fold[k][lane] = folded ? __fadd_rn(M.fold[k][lane], acc[k]) : acc[k];
-              acc[k] = 0.f;
-            }
-            folded = true;
-          }
-        }
       } else {
         // the first row of a piece may be another's too, a long row has sums
         // put aside, and a window of rows or scales may not reach the last
@@ -599,6 +591,17 @@ struct Walk {
               r = nr;
             }
           }
+        }
+      }
+      if constexpr (!ORDERED) {
+        // each group for itself: the others' rows may end in every step
+        if ((i & (kFold - 1)) == kFold - 1 && ends == 0) {
+#pragma unroll
+          for (int k = 0; k < P; ++k) {
+            M.fold[k][lane] = folded ? __fadd_rn(M.fold[k][lane], acc[k]) : acc[k];
+            acc[k] = 0.f;
+          }
+          folded = true;
         }
       }
       x = xn;
