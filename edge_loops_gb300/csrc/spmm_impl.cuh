@@ -72,6 +72,7 @@ struct Args {
   CarrySlot* flags;
   float* vec;  // num_ranges x kPassCols row-vector carries
   unsigned long long wait_ns;
+  int test_hooks;
 };
 
 // --------------------------------------------------------------- B elements
@@ -740,7 +741,7 @@ __global__ void __launch_bounds__(kTPB, kMinCtas) spmm_kernel(const Args a) {
         if (lane + 32 * q < a.n) __stcg(dst + lane + 32 * q, run[q]);
       __threadfence();
       __syncwarp();
-      if (lane == 0) st_release_u32(&a.flags[w].flag, tag);
+      if (lane == 0 && !(a.test_hooks & 1)) st_release_u32(&a.flags[w].flag, tag);
     }
     if (wait_row) {
       // row r0 began in range `first`: add the partials of ranges [first, w)
@@ -917,6 +918,7 @@ el_status launch(const SpmmCall& c, int schedule) {
   a.flags = c.ws.slots;
   a.vec = reinterpret_cast<float*>(c.scratch);
   a.wait_ns = c.wait_ns;
+  a.test_hooks = c.o.test_hooks;
   if (schedule == EL_SCHED_THREAD_MAPPED && c.n <= kNarrow) {
     a.n = (int)c.n;
     a.b_first = 0;
