@@ -535,10 +535,10 @@ struct Walk {
 #pragma unroll
         for (int j = 0; j < U; ++j) add(v[j], b[j], acc);
       } else {
-        // the first row of a piece may be another's too, a long row has sums
-        // put aside, and a window of rows or scales may not reach the last
-        // end: those go one by one
-        bool each = ends != 0 && (began || folded);
+        if (ends) unfold();
+        // the first row of a piece may be another's too, and a window of rows or
+        // scales may not reach the last end: those go one by one
+        bool each = ends != 0 && began;
         unsigned rw = 0u;
         if (!dense) {
           rw = bits_at(M.rowm, min(x - rs, nrows));
@@ -571,7 +571,6 @@ struct Walk {
             }
             add(M.val[slot][grp * G + j], bj, acc);
             if ((ends >> j) & 1u) {
-              unfold();
               if (began) {
                 if constexpr (!ORDERED) {
 #pragma unroll
