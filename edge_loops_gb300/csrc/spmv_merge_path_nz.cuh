@@ -267,8 +267,9 @@ __device__ __forceinline__ Acc<COMP> walk_rows(const Src& m, WarpSmem<COMP, KP>&
         const bool in = (unsigned)(ra + base + lane) < (unsigned)re && e <= hi;
         const unsigned b = __ballot_sync(kFullMask, in);
         const int cnt = b == kFullMask ? 32 : __ffs(~b) - 1;
-        const int el = (e <= hi ? max(e, lo) : hi) - lo;
-        int pe = __shfl_up_sync(kFullMask, el, 1);
+        // (-1 where an offset is below the tile: malformed, and not rising)
+        const int el = min(max(e, lo - 1), hi) - lo;
+        int pe = __shfl_up_sync(kFullMask, max(el, 0), 1);
         if (lane == 0) pe = prev;
         if (lane < cnt) {
           if (base > 0) S.re[base + lane] = el;  // the first 32 stay in el0
@@ -277,7 +278,7 @@ __device__ __forceinline__ Acc<COMP> walk_rows(const Src& m, WarpSmem<COMP, KP>&
         if (base == 0) el0 = el;
         X = base + cnt;
         if (cnt < 32 || X >= kMaxEnds) break;
-        prev = __shfl_sync(kFullMask, el, 31);
+        prev = __shfl_sync(kFullMask, max(el, 0), 31);
         base += 32;
         const int k = ra + base + 1 + lane;
         e = base == 32 && has_o2 ? o2 : k <= rows ? __ldg(m.offsets + k) : 0x7fffffff;
@@ -289,7 +290,7 @@ __device__ __forceinline__ Acc<COMP> walk_rows(const Src& m, WarpSmem<COMP, KP>&
     const float sc0 = scn;
     if (!fast && lane < X) S.re[lane] = el0;
     __syncwarp();
-    if (X >= kMaxEnds) hi = lo + S.re[kMaxEnds - 1];  // cut the tile at its 256th row end
+    if (X >= kMaxEnds) hi = lo + max(S.re[kMaxEnds - 1], 0);  // cut the tile at its 256th row end
     const int Y = hi - lo;
     if (X == 0 && Y == 0) {  // no progress possible: malformed offsets
       bad = true;
@@ -420,7 +421,7 @@ __device__ __forceinline__ Acc<COMP> walk_rows(const Src& m, WarpSmem<COMP, KP>&
       S.mw[lane] = 0u;  // only this lane reads it; the next tile writes it after a barrier
       // the lane's first row end (lane 0: a row closed at position 0, before any
       // nonzero of the tile, comes first)
-      const bool z = lane == 0 && X > 0 && S.re[0] == 0;
+      const bool z = lane == 0 && X > 0 && S.re[0] <= 0;
       const int k = z || mask == 0u ? 0 : S.kp[lane][__ffs(mask) - 1];
       Acc<COMP> run;
 #pragma unroll
@@ -487,6 +488,7 @@ __device__ __forceinline__ Acc<COMP> walk_rows(const Src& m, WarpSmem<COMP, KP>&
         cnt = 0;
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
+          bad |= e[u] < lo2;
           const unsigned b = __ballot_sync(kFullMask, e[u] <= lo2);
           const int c32 = b == kFullMask ? 32 : __ffs(~b) - 1;
           if (cnt == 32 * u) {

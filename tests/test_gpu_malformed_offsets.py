@@ -105,3 +105,22 @@ def test_spmm_flags_bad_offsets(cuda, kind, schedule):
              wait_limit_us=2000)
     torch.cuda.synchronize()
     assert ws.errors() & _lib.EL_FLAG_OFFSETS
+
+
+@pytest.mark.parametrize("kind", ["negative", "int min", "too large", "int max", "falls", "reversed",
+                                  "random"])
+@pytest.mark.parametrize("schedule,opts", [
+    ("merge_path", {}), ("merge_path", {"nz_per_lane": 8}), ("merge_path", {"nz_per_lane": 16}),
+    ("work_oriented", {"num_threads": 512}), ("work_oriented", {"num_threads": 128 * 304}),
+    ("group_mapped", {}), ("group_mapped", {"group_rows": 32})],
+    ids=lambda v: v if isinstance(v, str) else "-".join(f"{k}{x}" for k, x in v.items()) or "default")
+def test_spmv_flags_bad_offsets(cuda, kind, schedule, opts):
+    """An offset that falls or leaves [0, nnz], wherever it is."""
+    from edge_loops_gb300 import _lib, api
+    ws = api.Workspace()
+    x = torch.rand(COLS, device=cuda)
+    for seed in range(12):
+        A = matrix(kind, 6000, np.random.default_rng(seed), cuda)
+        api.spmv(A, x, schedule=schedule, workspace=ws, wait_limit_us=2000, **opts)
+        torch.cuda.synchronize()
+        assert ws.errors() & _lib.EL_FLAG_OFFSETS, seed
