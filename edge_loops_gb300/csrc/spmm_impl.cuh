@@ -177,9 +177,14 @@ __device__ __forceinline__ unsigned bits_at(const unsigned* m, int at) {
   return __funnelshift_r(m[at >> 5], m[(at >> 5) + 1], at & 31);
 }
 
-template <typename L, bool ORDERED>
+struct RowSmem {  // per warp, where it takes whole rows
+  int idx[2][32];
+  float val[2][32];
+};
+
+template <typename L, bool ORDERED, typename Sm_ = Smem<L, ORDERED>>
 struct Walk {
-  using Sm = Smem<L, ORDERED>;
+  using Sm = Sm_;
   static constexpr int G = L::G, U = L::U, NG = 32 / G, P = L::P, V = L::V, K = L::K;
   // (a block closes at most kBlock nonzeros beside its first row's)
   const Args& a;
@@ -253,10 +258,14 @@ struct Walk {
     }
   }
 
-  // One long row, nonzeros [b, e) in order, by the whole warp: the groups read
+  // One row, nonzeros [b, e) in order, by the whole warp: the groups read
   // the B rows of NG U nonzeros at once and add their products in turn, each
   // group to the sum the one before it hands on.
-  __device__ __forceinline__ void long_row(int row, int b, int e) {
+  // LEAN: the shorter code, for the walk, which it slows less (166,000 log-normal
+  // rows of 12, n = 16: 65 us lean, 78 not; a warp per row, BF16 B, n = 33, 5,000
+  // of them: 53 us lean, 27 not).
+  template <bool LEAN>
+  __device__ __forceinline__ void whole_row(int row, int b, int e) {
     float acc[P];
 #pragma unroll
     for (int k = 0; k < P; ++k) acc[k] = 0.f;
@@ -272,19 +281,31 @@ struct Walk {
       bad_col |= sl < U && y + mine < e && !ok;
       const int next = y + NG * U + mine;
       nz.load(a, sl < U && next < e, next);
+      const bool whole = !LEAN && __all_sync(kFullMask, ok || sl >= U);
       __syncwarp();
       BVec<L> bv[U][K];
+      if (whole) {
 #pragma unroll
-      for (int j = 0; j < U; ++j) {
-        const int c = M.idx[slot][grp * G + j];
+        for (int j = 0; j < U; ++j) {
+          const int c = M.idx[slot][grp * G + j];
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-          bv[j][k].zero();
-          if (c >= 0) bv[j][k].load(my_B[k] + (unsigned long long)(unsigned)c * a.ldb);
+          for (int k = 0; k < K; ++k)
+            bv[j][k].load(my_B[k] + (unsigned long long)(unsigned)c * a.ldb);
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < U; ++j) {
+          const int c = M.idx[slot][grp * G + j];
+#pragma unroll
+          for (int k = 0; k < K; ++k) {
+            bv[j][k].zero();
+            if (c >= 0) bv[j][k].load(my_B[k] + (unsigned long long)(unsigned)c * a.ldb);
+          }
         }
       }
+      const int groups = LEAN ? NG : min(NG, (e - y + U - 1) / U);  // with a nonzero of this step
 #pragma unroll 1
-      for (int g = 0; g < NG; ++g) {
+      for (int g = 0; g < groups; ++g) {
         if (grp == g) {  // a nonzero past the end adds 0 * 0 to a sum that is never -0
 #pragma unroll
           for (int j = 0; j < U; ++j) add(M.val[slot][grp * G + j], bv[j], acc);
@@ -677,7 +698,7 @@ __global__ void __launch_bounds__(kTPB, kMinCtas) spmm_kernel(const Args a) {
         if (rs >= re) break;
         const int b = min(max(__ldg(a.offsets + rs), ns), ne);
         ns = min(max(__ldg(a.offsets + rs + 1), b), ne);
-        walk.long_row(rs++, b, ns);
+        walk.template whole_row<true>(rs++, b, ns);
       }
     } else {
       if (d == d0) {
@@ -790,6 +811,56 @@ __global__ void __launch_bounds__(kTPB, kMinCtas) spmm_kernel(const Args a) {
   }
 }
 
+// --------------------------------------------------------------- few rows
+// ORDERED, a matrix of few rows: a warp per row, 32 / G x U of its B rows in
+// flight at once.  A row of 30 nonzeros is then one or two round trips; the
+// walk's range of a few rows is its split search, its row ends and a chain of
+// U nonzeros per step in one group of the warp, the other groups idle.  Up to
+// kFewRows rows per resident warp of the walk (3 where a lane holds 8 columns,
+// whose hand-over from group to group costs twice as much).  FP32 B, n = 8, the
+// walk / a warp per row: 5,276 rows of 38 11 / 7 us, 15,802 13-22 / 14, 52,644
+// 22 / 42; 13,346 of 15 10 / 7, 40,013 14 / 17; 15,013 of 4 7 / 6, 50,013
+// 9 / 15; 27-point stencil 8,000 rows 12 / 6, 21,952 15 / 15; log-normal rows of
+// 12, 16,679 27 / 22, 50,013 32 / 33.  BF16 B, n = 16 (8 columns per lane):
+// 8,000 stencil rows 14 / 9, 13,346 of 15 11 / 10, 15,802 of 38 17 / 21.
+constexpr int kFewRows = 5, kFewRowsWide = 3;
+template <typename L>
+__global__ void __launch_bounds__(kTPB, kMinCtas) warp_rows_kernel(const Args a) {
+  __shared__ RowSmem smem[kWarps];
+  Walk<L, true, RowSmem> walk(a, smem[threadIdx.x >> 5]);
+  const int nnz = (int)a.nnz;
+  const long long step = (long long)gridDim.x * kWarps;
+  auto bound = [&](long long r) { return __ldg(a.offsets + min(r, a.rows)); };
+  long long row = (long long)blockIdx.x * kWarps + (threadIdx.x >> 5);
+  int b = bound(row), e = bound(row + 1);
+  for (; row < a.rows; row += step) {  // warp-uniform
+    // the next row's bounds are in flight meanwhile
+    const int nb = bound(row + step), ne = bound(row + step + 1);
+    walk.bad_off |= b < 0 || e < b || e > nnz;
+    const int lo = min(max(b, 0), nnz);
+    walk.template whole_row<false>((int)row, lo, min(max(e, lo), nnz));
+    b = nb;
+    e = ne;
+  }
+  if (walk.bad_off) raise_flag(a.hdr, EL_FLAG_OFFSETS, 0);
+  if (walk.bad_col) raise_flag(a.hdr, EL_FLAG_INDEX_RANGE, 0);
+}
+
+template <typename L>
+bool few_rows(const SpmmCall& c) {
+  const long long warps = (long long)device_info(c.device).sm_count * kMinCtas * kWarps;
+  return c.A.rows <= warps * (L::P <= 4 ? kFewRows : kFewRowsWide);
+}
+
+template <typename L>
+el_status launch_warp_rows(const SpmmCall& c, const Args& a) {
+  const int per_sm = resident_ctas_per_sm((const void*)warp_rows_kernel<L>, kTPB, 0);
+  const long long most = (long long)(per_sm > 0 ? per_sm : 1) * device_info(c.device).sm_count;
+  const long long need = (a.rows + kWarps - 1) / kWarps;
+  warp_rows_kernel<L><<<(unsigned)(need < most ? need : most), kTPB, 0, c.stream>>>(a);
+  return cuda_status(cudaGetLastError(), "spmm launch");
+}
+
 // ------------------------------------------------------------- narrow B, C
 // thread_mapped with NC <= kNarrow columns: a thread per row, the row walked
 // once, W nonzeros' values and B elements in flight with the next W's
@@ -894,6 +965,7 @@ el_status launch_kernel(const SpmmCall& c, Args a) {
 template <typename BT, int V, int K, int G>
 el_status launch_pass(const SpmmCall& c, const Args& a, bool ordered) {
   using L = Lay<BT, V, K, G>;
+  if (ordered && few_rows<L>(c)) return launch_warp_rows<L>(c, a);
   return ordered ? launch_kernel<L, true>(c, a) : launch_kernel<L, false>(c, a);
 }
 
