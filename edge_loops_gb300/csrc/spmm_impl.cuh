@@ -326,9 +326,9 @@ struct Walk {
   // One block: rows [rs, re), at most kMaxRows, and nonzeros [ns, ne), the rows'
   // ends among them (not ORDERED: at most kMaxNz).  `inside`: row rs began before
   // nonzero ns.  z_out: row rs ends here without a nonzero.  ORDERED: stops
-  // before the first row that is long or whose offsets fall or leave [ns, ne], so
-  // that the rows before it have distinct ends in order; returns the row it
-  // stopped at.
+  // before the first row that is long, whose offsets fall or that ends before ns
+  // or kMaxNz past it, so that the rows before it end in order; returns the row
+  // it stopped at.
   // Leaves every piece's open row in M.open, with M.first, closed, has_pend.
   __device__ __forceinline__ int block(const int rs, int re, const int ns, int ne,
                                        const bool inside, bool& z_out) {
@@ -363,12 +363,12 @@ struct Walk {
         if (i0 + 32 * u >= nrows) break;
         const int i = i0 + 32 * u + lane, s = s4[u], e = e4[u];
         if constexpr (ORDERED) {
-          const int most = NG > 1 ? a.long_row : kMaxNz - kBlock;
-          const bool off = i < nrows && (s < ns || e < s || e > ne);
-          bad_off |= off;
+          const unsigned most = NG > 1 ? (unsigned)a.long_row : kMaxNz - kBlock;
           const unsigned lm = __ballot_sync(
-              kFullMask, i < nrows && (off || e - s > most || e - ns > kMaxNz));
+              kFullMask, i < nrows && ((unsigned)e - (unsigned)s > most ||  // or e < s
+                                       (unsigned)e - (unsigned)ns > (unsigned)kMaxNz));
           if (lm) {  // the block ends before this row
+            bad_off |= i < nrows && (s < ns || e < s || e > ne);
             const int q = __ffs(lm) - 1;
             nrows = i0 + 32 * u + q;
             ne = min(max(__shfl_sync(kFullMask, s, q), ns), ne);

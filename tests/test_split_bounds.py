@@ -145,7 +145,7 @@ def spmm_block(off, nnz, rs, re, ns, ne, inside, ordered, groups, u, long_row):
     if ordered:
         for i in range(nrows):
             s, e = int(off[rs + i]), int(off[rs + i + 1])
-            if s < ns or e < s or e > ne or e - s > long_row or e - ns > MAX_NZ:
+            if not 0 <= e - s <= long_row or not 0 <= e - ns <= MAX_NZ:
                 nrows, ne = i, min(max(s, ns), ne)
                 break
     ends, rowm, z_out = set(), [], False
