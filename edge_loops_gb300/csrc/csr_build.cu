@@ -299,11 +299,11 @@ __global__ void __launch_bounds__(kMoveThreads, 2)
   constexpr int kNone = -1;  // no entry (as a heavy place: past every one)
   auto window = [](int e) { return e == kNone ? -1 : (int)(((unsigned)e & ~kHeavy) >> LOGW); };
   for (int i = threadIdx.x; i < windows; i += T) count[i] = 0u;
-  __syncthreads();
   const long long base = (long long)blockIdx.x * kMoveTile;
   int est[P], c[P];
   float v[P];
   unsigned at[P];
+  const unsigned full = *const_cast<volatile unsigned*>(flags + 1);
 #pragma unroll
   for (int i = 0; i < P; ++i) {
     const long long k = base + i * T + threadIdx.x;
@@ -311,6 +311,8 @@ __global__ void __launch_bounds__(kMoveThreads, 2)
     c[i] = k < nnz ? __ldcs(ci + k) : -1;
     v[i] = k < nnz ? __ldcs(vin + k) : 0.f;
   }
+  // a window is full: the radix sort it is, so nothing more is moved
+  if (__syncthreads_or(full != 0u)) return;
 #pragma unroll
   for (int i = 0; i < P; ++i) {
     const int r = est[i];
@@ -378,7 +380,7 @@ __global__ void __launch_bounds__(kMoveThreads, 2)
     const unsigned slot = count[b] + k;
     if (slot < (unsigned)Wn::kCap)
       recs[(size_t)b * Wn::kCap + slot] = r;
-    else
+    else if (slot == (unsigned)Wn::kCap)  // one store per window, not one per entry
       flags[1] = 1u;
   }
 }
@@ -559,9 +561,9 @@ __global__ void __launch_bounds__(Win<LOGW>::kThreads, 1)
 // The two ways.  A status, and *done = whether the arrays are written.
 template <int LOGW>
 el_status window_sort(el_workspace* w, const el_coo* coo, int32_t* offsets, int32_t* indices,
-                      float* values, cudaStream_t s, int sms, bool* done) {
+                      float* values, cudaStream_t s, int sms, bool* done, bool* checked) {
   using Wn = Win<LOGW>;
-  *done = false;
+  *done = *checked = false;
   const long long nnz = coo->nnz, rows = coo->rows, n = rows + 1;
   const int windows = (int)((nnz + Wn::W - 1) / Wn::W);
   const long long blocks = (n + kScan - 1) / kScan;
@@ -615,6 +617,7 @@ el_status window_sort(el_workspace* w, const el_coo* coo, int32_t* offsets, int3
   if (e != cudaSuccess) return cuda_status(e, "el_csr_from_coo: move");
   if (h[0]) return fail(EL_ERR_MALFORMED_CSR, "COO entry outside %lld x %lld",
                         (long long)coo->rows, (long long)coo->cols);
+  *checked = true;
   if (h[1]) return EL_OK;  // a window is full
   e = cudaFuncSetAttribute(window_sort_kernel<LOGW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            Wn::kSmem);
@@ -625,8 +628,9 @@ el_status window_sort(el_workspace* w, const el_coo* coo, int32_t* offsets, int3
   return cuda_status(cudaGetLastError(), "el_csr_from_coo: sort");
 }
 
+// `checked`: every entry is known to be in range.
 el_status radix_sort(el_workspace* w, const el_coo* coo, int32_t* offsets, int32_t* indices,
-                     float* values, cudaStream_t s, int sms) {
+                     float* values, cudaStream_t s, int sms, bool checked) {
   const long long nnz = coo->nnz;
   const int cbits = bits_for(coo->cols > 0 ? coo->cols : 1);
   // temporaries in the workspace's staging memory:
@@ -660,8 +664,10 @@ el_status radix_sort(el_workspace* w, const el_coo* coo, int32_t* offsets, int32
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_status(e, "el_csr_from_coo: keys");
   unsigned h_bad = 0;
-  e = cudaMemcpyAsync(&h_bad, bad, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (!checked) {
+    e = cudaMemcpyAsync(&h_bad, bad, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  }
   if (e != cudaSuccess) return cuda_status(e, "el_csr_from_coo: check");
   if (h_bad) return fail(EL_ERR_MALFORMED_CSR, "COO entry outside %lld x %lld",
                          (long long)coo->rows, (long long)coo->cols);
@@ -713,12 +719,13 @@ extern "C" el_status el_csr_from_coo(el_workspace* ws, const el_coo* coo, int32_
   // Small windows give few entries enough CTAs; large ones keep the move's
   // atomics (entries / 4096 x windows) few: 2M entries 197 us by windows of
   // 2048, 3M 193 us by windows of 8192.
-  bool done = false;
+  bool done = false, checked = false;
   if (nnz >= Win<11>::W && coo->rows <= 2 * nnz + (1 << 20) &&
       nnz <= (long long)kMaxWindows * Win<13>::W) {
-    st = nnz <= kSmallNnz ? window_sort<11>(w, coo, offsets, indices, values, s, sms, &done)
-                          : window_sort<13>(w, coo, offsets, indices, values, s, sms, &done);
+    st = nnz <= kSmallNnz
+             ? window_sort<11>(w, coo, offsets, indices, values, s, sms, &done, &checked)
+             : window_sort<13>(w, coo, offsets, indices, values, s, sms, &done, &checked);
     if (st != EL_OK || done) return st;
   }
-  return radix_sort(w, coo, offsets, indices, values, s, sms);
+  return radix_sort(w, coo, offsets, indices, values, s, sms, checked);
 }
