@@ -34,9 +34,9 @@ static_assert(sizeof(WsHeader) == 64, "header is one 64-byte line");
 
 struct CarrySlot {  // one partial row sum handed to a later CTA
   float sum;
-  float comp;
   unsigned int flag;  // == epoch_tag(epoch of the publishing launch)
-  unsigned int pad;
+  float comp;
+  unsigned int flag2;  // the same for comp, where publish_carry wrote it
 };
 
 // Never 0 (the value of a slot nobody ever published).
@@ -213,6 +213,34 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
 
 __device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// A carry whose sum and tag (and, compensated, comp and tag) are one 8-byte word
+// each, written and read by one access: the reader needs no second read after
+// the tag (a row over 3648 ranges, whose last one reads 114 carries per lane one
+// after the other: 56 -> LBUS us).
+template <bool COMP>
+__device__ __forceinline__ void publish_carry(CarrySlot* s, float sum, float comp, unsigned tag) {
+  auto put = [&](void* p, float v) {
+    const unsigned long long w = (unsigned long long)tag << 32 | __float_as_uint(v);
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
+  };
+  if (COMP) put(&s->comp, comp);
+  put(&s->sum, sum);
+}
+// Whether the carry is there (then in sum and comp).
+template <bool COMP>
+__device__ __forceinline__ bool take_carry(const CarrySlot* s, unsigned tag, float* sum,
+                                           float* comp) {
+  auto get = [](const void* p) {
+    unsigned long long w;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(p) : "memory");
+    return w;
+  };
+  const unsigned long long a = get(&s->sum), b = COMP ? get(&s->comp) : 0ull;
+  *sum = __uint_as_float((unsigned)a);
+  *comp = __uint_as_float((unsigned)b);
+  return (unsigned)(a >> 32) == tag && (!COMP || (unsigned)(b >> 32) == tag);
 }
 
 // Named barrier over the first `nthreads` threads of the CTA (the consumer

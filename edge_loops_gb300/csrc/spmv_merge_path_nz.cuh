@@ -536,22 +536,34 @@ __device__ __forceinline__ Acc<COMP> look_back(const Args& a, long long gfirst, 
   Acc<COMP> acc;
   ok = true;
   if (gfirst < 0) gfirst = 0;  // malformed offsets
-  for (long long kk = gfirst + lane; kk < g && kk < a.ws.nslots; kk += 32) {
-    CarrySlot* sl = a.ws.slots + kk;
-    if (ld_acquire_u32(&sl->flag) != tag) {
-      const uint64_t t0 = global_timer_ns();
-      while (ld_acquire_u32(&sl->flag) != tag) {
-        if (global_timer_ns() - t0 > a.wait_ns) {
-          ok = false;
-          break;
+  constexpr int kAhead = 4;  // carries read at once, added in order
+  const long long end = min(g, a.ws.nslots);
+  for (long long k0 = gfirst + lane; k0 < end && ok; k0 += 32 * kAhead) {
+    float sum[kAhead], comp[kAhead];
+    bool have[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      have[u] = k0 + 32 * u < end &&
+                take_carry<COMP>(a.ws.slots + k0 + 32 * u, tag, &sum[u], &comp[u]);
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const long long kk = k0 + 32 * u;
+      if (kk >= end || !ok) break;
+      if (!have[u]) {
+        const uint64_t t0 = global_timer_ns();
+        while (!take_carry<COMP>(a.ws.slots + kk, tag, &sum[u], &comp[u])) {
+          if (global_timer_ns() - t0 > a.wait_ns) {
+            ok = false;
+            break;
+          }
+          __nanosleep(100);
         }
-        __nanosleep(100);
+        if (!ok) break;
       }
+      Acc<COMP> pv;
+      pv.set(sum[u], comp[u]);
+      acc.add(pv);
     }
-    if (!ok) break;
-    Acc<COMP> pv;
-    pv.set(__ldcg(&sl->sum), __ldcg(&sl->comp));
-    acc.add(pv);
   }
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) {
@@ -637,10 +649,7 @@ __device__ __forceinline__ void run_range(const Args& a, SmemT& S, const int war
       if ((long long)re == a.rows && (long long)off_re != a.nnz)
         raise_flag(hdr, EL_FLAG_NNZ_MISMATCH, (unsigned)re);
       if (ne > max(off_re, ns) && g < a.ws.nslots && !(a.test_hooks & 1)) {
-        CarrySlot* sl = a.ws.slots + g;
-        sl->sum = carry.s;
-        sl->comp = carry.comp();
-        st_release_u32(&sl->flag, tag);
+        publish_carry<COMP>(a.ws.slots + g, carry.s, carry.comp(), tag);
       }
     }
     __syncwarp();

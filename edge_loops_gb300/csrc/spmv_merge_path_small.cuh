@@ -145,10 +145,7 @@ __global__ void __launch_bounds__(kSmTPB) merge_path_small_kernel(const Args a) 
     if (ne > lo) {
       const float s = warp_sum(min(lo - n0, len), len);
       if (lane == 0 && g < a.ws.nslots && !(a.test_hooks & 1)) {
-        CarrySlot* const sl = a.ws.slots + g;
-        sl->sum = s;
-        sl->comp = 0.f;
-        st_release_u32(&sl->flag, tag);
+        publish_carry<false>(a.ws.slots + g, s, 0.f, tag);
       }
     }
   }
