@@ -484,10 +484,10 @@ struct Walk {
 #pragma unroll
     for (int k = 0; k < P; ++k) acc[k] = 0.f;
     bool has_pend = false;
-    // a row's sum is put aside in every kFold-th step unless the row's group has a
-    // row end in it: short chains of additions, for the rounding error (a row
-    // that begins in such a step waits for the next: at most (kFold + 1) U - 1
-    // nonzeros in one chain)
+    // a row's sum is put aside before every kFold-th step unless its group has a
+    // row end in that step: short chains of additions, for the rounding error
+    // (at most (kFold + 1) U - 1 nonzeros).  Each group for itself: the others'
+    // rows may end in every step.
     bool folded = false;
     auto unfold = [&]() {
       if constexpr (!ORDERED) {
@@ -501,8 +501,7 @@ struct Walk {
     float* crow = a.C + (long long)x * a.ldc + L::column(sl, 0);
     float scn = scale ? __ldg(scale + min(x + sl, (int)a.rows - 1)) : 1.f;
     unsigned ends = step_ends(y);
-#pragma unroll 1
-    for (int i = 0; i < steps; ++i) {
+    auto step = [&](int i) {
       const int slot = i & 1;
       const bool ok = (unsigned)nz.c < (unsigned long long)a.cols;
       const bool in = y + sl < ye;
@@ -556,7 +555,6 @@ struct Walk {
 #pragma unroll
         for (int j = 0; j < U; ++j) add(v[j], b[j], acc);
       } else {
-        if (ends) unfold();
         // the first row of a piece may be another's too, and a window of rows or
         // scales may not reach the last end: those go one by one
         bool each = ends != 0 && began;
@@ -567,7 +565,12 @@ struct Walk {
           each |= ends != 0 && (!(rw & 1u) || __popc(rw) <= ne_ ||
                                 (scale && __popc(rw & (kFullMask >> (32 - G))) < ne_));
         }
-        if (!__any_sync(kFullMask, each)) {
+        bool any_each = __any_sync(kFullMask, each || (folded && ends != 0));
+        if (any_each) {  // a sum put aside is taken up before the step of its row's end
+          if (ends) unfold();
+          any_each = __any_sync(kFullMask, each);
+        }
+        if (!any_each) {
           if (dense) {
             if (scale)
               sums<false, true>(b, v, ends, 0u, sc, acc, crow);
@@ -614,9 +617,14 @@ struct Walk {
           }
         }
       }
+      x = xn;
+      y = min(y + U, ye);
+      ends = step_ends(y);
+    };
+#pragma unroll 1
+    for (int i0 = 0; i0 < steps; i0 += kFold) {
       if constexpr (!ORDERED) {
-        // each group for itself: the others' rows may end in every step
-        if ((i & (kFold - 1)) == kFold - 1 && ends == 0) {
+        if (i0 > 0 && ends == 0) {
 #pragma unroll
           for (int k = 0; k < P; ++k) {
             M.fold[k][lane] = folded ? __fadd_rn(M.fold[k][lane], acc[k]) : acc[k];
@@ -625,9 +633,9 @@ struct Walk {
           folded = true;
         }
       }
-      x = xn;
-      y = min(y + U, ye);
-      ends = step_ends(y);
+      const int i1 = min(i0 + kFold, steps);
+#pragma unroll 1
+      for (int i = i0; i < i1; ++i) step(i);
     }
     unfold();
     __syncwarp();
