@@ -25,10 +25,12 @@
 //
 // Measured, whole call: 15.4M shuffled entries of a 2^20-row power-law matrix
 // 1128 us by the radix sort of a 51-bit key (7 passes of 120 us, values
-// gathered 102 us, offsets searched 33 us), 682 us by the window sort (count
-// 137, sums 38, move 240, sort 250 us).  Uniform entries: 20,000 145 -> 83 us,
-// 1M 221 -> 143, 8M 728 -> 400; 8M within 300 columns of 2^20 599 -> 386;
-// 13.5M of a stencil 1054 -> 659.
+// gathered 102 us, offsets searched 33 us), 627 us by the window sort (count
+// 87, sums 12, move 242, sort 278 us).  Uniform entries in rows of 15: 200,000
+// 147 -> 70 us, 2M 275 -> 147, 8M 669 -> 333, 15M 1124 -> 638.  A twentieth of the
+// entries in one row's few columns, which overfills a window and goes to the
+// radix sort of a 40-bit key: 200,000 147 -> 143, 2M 273 -> 274, 8M 668 -> 620, 15M
+// 1120 -> 1027.
 #include <algorithm>
 
 #include <cub/device/device_radix_sort.cuh>

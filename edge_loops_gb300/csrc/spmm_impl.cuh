@@ -876,8 +876,14 @@ el_status launch_warp_rows(const SpmmCall& c, const Args& a) {
 // rows of a banded matrix share them in L1, and the row ends of the walk above
 // cost as much as for wide rows.  2M nonzeros, FP32, walk / thread per row:
 // 27-point stencil n = 1 29 / 10 us, n = 4 28 / 14; n = 4 in log-normal rows of
-// 4 59 / 32, uniform rows of 38 28 / 30, log-normal rows of 38 77 / 98.  From 6
-// columns on the walk is faster.
+// 4 59 / 32, uniform rows of 38 28 / 30, log-normal rows of 38 77 / 98.  The line
+// is by n alone: where rows are long the thread per row loses up to a quarter,
+// where they are short the walk loses half, and how the lengths vary, which
+// decides between them from 6 columns on (n = 6: stencil 27 / 12, uniform rows of
+// 38 25 / 34, log-normal rows of 27 76 / 106, of 4 65 / 43), is not known here.  So
+// from 6 columns on the walk keeps rows of every length balanced, and a stencil
+// of more rows than the warp per row takes is slower than by a thread per row
+// (22,000 rows, n = 6: 16 / 6).
 constexpr int kNarrow = 5;
 template <typename VT, typename BT, int NC>
 __global__ void __launch_bounds__(256, 3) thread_rows_kernel(const Args a) {

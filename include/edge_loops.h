@@ -144,9 +144,12 @@ typedef struct el_spmv_opts {
                                 thread and tile (1..16, tile = 256 x this);
                                 variant 0 and work_oriented: unused */
   int32_t threads_per_row;   /* thread_mapped: 1,2,4,8,16,32 lanes per row */
-  int32_t group_rows;        /* group_mapped: rows per group: 32 (one warp
-                                per group, the reference's warp_mapped) or
-                                threads_per_block (block_mapped) */
+  int32_t group_rows;        /* group_mapped: rows per group: 32 (the
+                                reference's warp_mapped) or
+                                threads_per_block (block_mapped).  A warp
+                                takes whole rows, 128 at a time (256 for
+                                groups of 256, fewer on small matrices),
+                                so 32 and 128 run the same launch */
   int64_t num_threads;       /* work_oriented: threads of the even split,
                                 a multiple of 128 (the reference uses
                                 2 x SMs x 128); 0 = 32 per resident warp.
@@ -156,8 +159,8 @@ typedef struct el_spmv_opts {
   int32_t max_ctas;          /* cap on persistent grids (0 = resident) */
   int32_t wait_limit_us;     /* bound on every device-side wait (0 = 2 s) */
   int32_t test_hooks;        /* testing only, 0 in normal use: bit 0 makes
-                                merge_path ranges skip publishing their row
-                                carries, so a range that needs one waits until
+                                merge_path (SpMM too) and work_oriented
+                                ranges skip publishing their row carries, so a range that needs one waits until
                                 wait_limit_us and reports EL_FLAG_TIMEOUT */
   int32_t variant;           /* merge_path kernel (same results within the
                                 FP32 bound, deterministic):
